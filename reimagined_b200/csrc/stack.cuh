@@ -101,7 +101,7 @@ cudaError_t allow_smem(Kernel kernel, size_t bytes, bool (&done)[64]) {
     return e;
 }
 
-// ---- dense.cu / dense_tcgen05.cu: y = W x + b with bf16 weights ------------------------------------------------
+// ---- dense.cu / dense_rows.cu / dense_tcgen05.cu / dense_split.cu: y = W x + b with bf16 weights ------------------------------------------------
 struct DenseCall {
     const void* x;           // activations, the precision's type
     const bf16* w;           // [N, K], ldw between rows (0: K)
@@ -119,12 +119,14 @@ struct DenseCall {
     long long batch_w, batch_x, batch_out;
     const float* gate;
 };
-enum DenseRoute { kDenseAuto = 0, kDenseSimt = 1, kDenseGemv = 2, kDenseTensor = 3, kDenseRows = 4 };
+enum DenseRoute { kDenseAuto = 0, kDenseSimt = 1, kDenseGemv = 2, kDenseTensor = 3, kDenseRows = 4, kDenseSplit = 5 };
 int launch_dense(int precision, int route, const DenseCall& c, cudaStream_t st);
 bool dense_rows_supported(const DenseCall& c);
 cudaError_t launch_dense_rows(const DenseCall& c, cudaStream_t st);
 bool dense_tensor_supported(const DenseCall& c);
 cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st);
+bool dense_split_supported(const DenseCall& c);
+cudaError_t launch_dense_split(const DenseCall& c, cudaStream_t st);
 
 // ---- stack_glue.cu ----------------------------------------------------------------------------------------------
 struct DepthNorm {

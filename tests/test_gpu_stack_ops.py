@@ -107,6 +107,40 @@ def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
     assert_close(f64(out), want, 4e-3 if precision else 3e-6)
 
 
+@pytest.mark.parametrize("m,k,n,ff,shift", [(5, 8, 1, 1, 0), (127, 72, 65, 33, 0), (129, 512, 64, 96, 1), (16, 1032, 130, 250, 0), (257, 4096, 63, 31, 0), (6, 1088, 12900, 6500, 0)])
+def test_dense_fp32_in_three_pieces(cuda, stack_lib, m, k, n, ff, shift):
+    """fp32 rows on the tensor cores: one to eight shares of K, rows of x that start on 16 bytes and that do not, gated pairs, and
+    rows with infinities, NaN and numbers near the end of the range, which have no three pieces."""
+    from reimagined_b200.stack import StackEngine
+    torch, rng = cuda, np.random.default_rng(m + n)
+    b = Buf(torch)
+    x = torch.as_tensor(rng.standard_normal((m, k + shift)), dtype=torch.float32).cuda()
+    w, gate, up = (torch.as_tensor(rng.standard_normal((r, k)), dtype=torch.float32).bfloat16() for r in (n, ff, ff))
+    bias, res = rng.standard_normal(n), rng.standard_normal((m, n)).astype(np.float32)
+    # a sum of a slab drops less than 2^-22 of the numbers added up, eight times; the same again for rounding
+    bound = 2.0 ** -18 * (x[:, :k].abs().double() @ w.cuda().abs().double().T + 8.0)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    view = b.view(w, bias)
+    call = lambda: stack_lib.tbl_dense_forward(C.byref(view), 0, 0, x.data_ptr(), k + shift, m, b.f32(res), out.data_ptr(), stream(torch))
+    assert call() == 0
+    want = x[:, :k].double() @ w.cuda().double().T + torch.as_tensor(bias).cuda().float().double() + torch.as_tensor(res).cuda().double()
+    assert bool(((out.double() - want).abs() <= bound).all())
+    paired = b.view(StackEngine._paired(None, gate, up))
+    h = torch.full((m, ff), float("nan"), device="cuda")
+    assert stack_lib.tbl_gated_dense_forward(C.byref(paired), 0, 0, x.data_ptr(), k + shift, m, ff, h.data_ptr(), stream(torch)) == 0
+    gw, uw = (x[:, :k].double() @ t.cuda().double().T for t in (gate, up))
+    assert_close(f64(h), (torch.nn.functional.silu(gw) * uw).cpu().numpy(), 3e-6)
+    x[1, 3], x[2, 0], x[4, 5] = float("inf"), float("nan"), 3.4e38
+    assert call() == 0
+    got, plain = out.clone(), torch.empty_like(out)
+    assert stack_lib.tbl_dense_forward(C.byref(view), 0, SIMT, x.data_ptr(), k + shift, m, b.f32(res), plain.data_ptr(), stream(torch)) == 0
+    same = (got == plain) | (got.isnan() & plain.isnan())
+    near = (got.double() - plain.double()).abs() <= 2.0 ** -18 * (x[:, :k].abs().double() @ w.cuda().abs().double().T + 8.0)
+    assert bool((same | near).all()) and bool(got[2].isnan().all())
+    assert bool((same[1]).all())
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 # ---- norm and depth average -----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("rows,width,count", [(1, 512, 1), (3, 1000, 12), (40, 90, 5), (2, 4100, 19), (33, 516, 9)])
