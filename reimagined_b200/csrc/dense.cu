@@ -224,10 +224,15 @@ bool gemv_supported(const DenseCall& c) {
     return c.M <= kGemvMaxRows && sizeof(float) * c.M * c.K <= kGemvMaxSmem && (c.K % 4 == 0 || c.M == 1);
 }
 
-// Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 16 rows, on narrow layers (too few tiles for
-// the GEMM to fill the GPU) longer.
+// Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 16 rows, except that more than eight rows of a
+// long K are better shared out (16 x 12288 x 4096: 32 and 23 us; 8 x 6144 x 2048: 9 and 12), and on small matrices
+// longer (32 x 2048 x 2048: 6.4 and 9.2 us, 32 x 4096 x 4096: 20 and 12, 64 x 1024 x 1024: 6.2 and 6.4, 64 x 2048 x 2048:
+// 10.1 and 8.8).
 bool rows_pay(const DenseCall& c) {
-    return c.batch > 0 || c.M <= 16 || static_cast<long long>(c.M) * c.N <= 32 * 4096;
+    const long long size = static_cast<long long>(c.N) * c.K;
+    if (c.batch > 0 || c.M <= 8) return true;
+    if (c.M <= 16) return c.K < 2LL * c.N || size < (12 << 20);
+    return c.M <= 32 ? size <= (10 << 20) : c.M * size <= (128 << 20);
 }
 
 }  // namespace

@@ -18,6 +18,7 @@
 // Every wait is bounded: on a timeout the role records the status word and falls through to the common exit.
 #include <cuda.h>
 
+#include "shares.cuh"
 #include "stack.cuh"
 #include "tc05.cuh"
 
@@ -47,17 +48,6 @@ struct Params {
     int tma_x, vec_out;      // rows of x start on 16 bytes / outputs take 16-byte accesses
     int* status;
 };
-
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 peer_load(uint32_t addr, int rank) {
-    uint32_t a;
-    float4 v;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-    return v;
-}
 
 // high halves of two words: the bf16 numbers nearest to them towards zero, packed
 __device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
@@ -243,58 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
     // ---------------- all shares' sums, a part of the rows per CTA ----------------
     pdl_wait();
     if (p.split > 1) cluster_sync_all(); else __syncthreads();
-    const bool pair = c.pair_cols > 0;
-    const int rows = min(BM, c.M - m0), each = (rows + p.split - 1) / p.split;
-    const int r0 = share * each, r1 = min(rows, r0 + each);
-    const int groups = pair ? BN / 8 : BN / 4;             // of four output columns
-    const int ncols = pair ? c.pair_cols : c.N;
-    const Activation act = activation_of(c.act);
-    const uint32_t sums = smem_u32(smem);
-    auto total = [&](int r, int col) {
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int k = 0; k < p.split; ++k) {
-            const float4 a = peer_load(sums + 4 * (r * LDS + col), k);
-            v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
-        }
-        return v;
-    };
-    for (int e = threadIdx.x; e < (r1 - r0) * groups; e += kThreads) {
-        const int r = r0 + e / groups, gq = e % groups, m = m0 + r;
-        const int col = pair ? gq / 8 * 64 + gq % 8 * 4 : 4 * gq;            // of the (first) weight row within the tile
-        const int row_w = tn * BN + col, n = pair ? tn * (BN / 2) + 4 * gq : row_w;
-        if (n >= ncols) continue;
-        const float4 t = total(r, col);
-        float v[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (n + j >= ncols) continue;
-            v[j] = checked(c, m, row_w + j, v[j]);
-            if (c.bias) v[j] += __ldg(c.bias + row_w + j);
-        }
-        if (pair) {
-            const float4 tu = total(r, col + 32);
-            const float u[4] = {tu.x, tu.y, tu.z, tu.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (n + j >= ncols) continue;
-                float up = checked(c, m, row_w + 32 + j, u[j]);
-                if (c.bias) up += __ldg(c.bias + row_w + 32 + j);
-                v[j] = activate(act, v[j]) * up;
-            }
-        }
-        const size_t o = static_cast<size_t>(m) * c.ldo + n;
-        if (p.vec_out) {
-            if (c.residual) {
-                const float4 res = *reinterpret_cast<const float4*>(c.residual + o);
-                v[0] += res.x; v[1] += res.y; v[2] += res.z; v[3] += res.w;
-            }
-            *reinterpret_cast<float4*>(c.out_f32 + o) = make_float4(v[0], v[1], v[2], v[3]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (n + j < ncols) c.out_f32[o + j] = c.residual ? c.residual[o + j] + v[j] : v[j];
-        }
-    }
+    finish_shares<BN, LDS, kThreads>(c, smem_u32(smem), p.split, share, tn, m0, BM, p.vec_out, [&](int m, int n, float v) { return checked(c, m, n, v); });
     // nobody leaves while a neighbour may still read its sums; then the allocating warp releases TMEM
     tc_fence_before();
     if (p.split > 1) cluster_sync_all(); else __syncthreads();
@@ -317,18 +256,10 @@ cudaError_t launch_bn(Params p, cudaStream_t st) {
     const int tiles_m = ceil_div(c.M, BM), tiles_n = ceil_div(c.N, BN), kblocks = ceil_div(c.K, BKE);
     // shares of K until the SMs are taken, of at least four blocks each
     p.split = 1;
-    while (p.split < kMaxSplit && 2LL * p.split * tiles_m * tiles_n <= kNumSm && kblocks >= 8 * p.split) p.split *= 2;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(tiles_n * p.split, tiles_m); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem_for(BN); cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 2;
-    e = cudaLaunchKernelEx(&cfg, dense_split_kernel<BN>, mx, mb, p);
-    note_launch();
-    return e;
+    while (p.split < kMaxSplit && kblocks >= 8 * p.split &&
+           2LL * p.split * tiles_m * tiles_n <= cluster_room(dense_split_kernel<BN>, 2 * p.split, kThreads, smem_for(BN)))
+        p.split *= 2;
+    return launch_dependent_cluster(dense_split_kernel<BN>, dim3(tiles_n * p.split, tiles_m), p.split, dim3(kThreads), smem_for(BN), st, mx, mb, p);
 }
 
 }  // namespace

@@ -2,7 +2,8 @@
 // gemm_tcgen05.cu, with the same roles and the same operand geometry (a stage is 128 bytes of K per row, i.e. 64
 // bf16, in the 128-byte-swizzled K-major layout TMA writes; an MMA takes 32 bytes of K).
 //
-// One persistent CTA per SM, ten warps: TMA producer, MMA issuer (tcgen05.mma kind::f16, fp32 accumulators in TMEM,
+// One persistent CTA per SM (or, where the tiles would leave SMs idle, a cluster of CTAs per tile that share its K range and
+// finish it together), ten warps: TMA producer, MMA issuer (tcgen05.mma kind::f16, fp32 accumulators in TMEM,
 // two buffers of BN columns), eight epilogue warps.  128 x BN tiles; the two accumulators double-buffer tiles.  (256 x
 // 256 tiles, which the int8 kernel uses for large problems, gain nothing here: these epilogues -- residual, gated pair --
 // are longer, and a tall tile cannot hide them.)
@@ -13,6 +14,7 @@
 // TMEM is released.
 #include <cuda.h>
 
+#include "shares.cuh"
 #include "stack.cuh"
 #include "tc05.cuh"
 
@@ -28,6 +30,7 @@ constexpr int BKE = BKB / 2;        // the same in elements
 constexpr int kGroupM = 16;         // row tiles per group of the tile walk
 constexpr int kMaxStages = 8;
 constexpr int kEpiWarps = 8;
+constexpr int kMaxSplit = 4;
 constexpr int kThreads = 32 * (2 + kEpiWarps);
 
 __host__ __device__ constexpr int stages_for(int bn) { return bn >= 256 ? 4 : (bn >= 128 ? 6 : 8); }
@@ -38,6 +41,7 @@ constexpr size_t smem_for(int bn) {
 struct Params {
     DenseCall c;
     int tiles_m, tiles_n;
+    int split;              // shares of K = CTAs of a cluster (SHARED kernel)
     int vec;                // outputs (and residual) take 4-column vector accesses
     int* status;
 };
@@ -102,9 +106,10 @@ __device__ __forceinline__ void store_block(const Params& p, const uint8_t* stag
     }
 }
 
-template <int BN, bool RES>
+// SHARED: a CTA takes one share of the K range of one tile, the CTAs of a cluster finish the tile together.
+template <int BN, bool RES, bool SHARED>
 __global__ void __launch_bounds__(kThreads, 1)
-dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Params p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     constexpr int kStages = stages_for(BN);
@@ -112,6 +117,8 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     constexpr int kBBytes = BN * BKB;
     constexpr int kStageBytes = kABytes + kBBytes;
     constexpr uint32_t kTmemCols = 2 * BN;
+    constexpr int LDS = BN + 4;                                        // floats per row of a share's sums
+    static_assert(!SHARED || sizeof(float) * BM * LDS <= kStages * kStageBytes, "the sums take the stages' place");
     uint8_t* epi_stage = smem + kStages * kStageBytes;                 // 8 warps x 4 KB
     uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + kEpiWarps * 4096);
     uint64_t* empty = full + kMaxStages;
@@ -120,7 +127,10 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kblocks = (p.c.K + BKE - 1) / BKE;
+    const int all_blocks = (p.c.K + BKE - 1) / BKE, per = SHARED ? (all_blocks + p.split - 1) / p.split : all_blocks;
+    const int share = SHARED ? blockIdx.x % p.split : 0, first = SHARED ? blockIdx.x / p.split : blockIdx.x;
+    const int stride = SHARED ? p.tiles_m * p.tiles_n : gridDim.x;     // SHARED: this tile only
+    const int kb0 = SHARED ? min(all_blocks, share * per) : 0, kblocks = SHARED ? min(all_blocks, kb0 + per) - kb0 : all_blocks;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -138,6 +148,17 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
+    // the weights of the first stages do not depend on the kernel before this one
+    int early = 0;
+    if (warp == 0) {
+        int row0, tn;
+        if (!p.c.w_computed && decode_tile(p, first, row0, tn)) early = min(kStages, kblocks);
+        if (lane == 0)
+            for (int s = 0; s < early; ++s) {
+                mbar_arrive_expect_tx(&full[s], kStageBytes);
+                tma_load_2d(smem + s * kStageBytes + kABytes, &map_b, (kb0 + s) * BKE, tn * BN, &full[s]);
+            }
+    }
     pdl_wait();
 
     if (warp == 0) {
@@ -145,7 +166,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (lane == 0) {
             int it = 0, row0, tn;
             bool alive = true;
-            for (int tile = blockIdx.x; alive && decode_tile(p, tile, row0, tn); tile += gridDim.x) {
+            for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride) {
                 for (int kb = 0; kb < kblocks; ++kb, ++it) {
                     const int s = it % kStages;
                     if (it >= kStages) {
@@ -153,9 +174,9 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         if (!alive) break;
                     }
                     uint8_t* a_dst = smem + s * kStageBytes;
-                    mbar_arrive_expect_tx(&full[s], kStageBytes);
-                    tma_load_2d(a_dst, &map_a, kb * BKE, row0, &full[s]);
-                    tma_load_2d(a_dst + kABytes, &map_b, kb * BKE, tn * BN, &full[s]);
+                    if (it >= early) mbar_arrive_expect_tx(&full[s], kStageBytes);
+                    tma_load_2d(a_dst, &map_a, (kb0 + kb) * BKE, row0, &full[s]);
+                    if (it >= early) tma_load_2d(a_dst + kABytes, &map_b, (kb0 + kb) * BKE, tn * BN, &full[s]);
                 }
             }
         }
@@ -165,7 +186,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const uint32_t idesc = idesc_bf16(BN);
             int it = 0, local = 0, row0, tn;
             bool alive = true;
-            for (int tile = blockIdx.x; alive && decode_tile(p, tile, row0, tn); tile += gridDim.x, ++local) {
+            for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride, ++local) {
                 const int buf = local & 1;
                 if (local >= 2) {
                     alive = mbar_wait_bounded(&tmem_empty[buf], ((local >> 1) - 1) & 1, p.status);
@@ -185,8 +206,29 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         umma_f16(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), idesc, (kb | kk) != 0 ? 1u : 0u);
                     umma_commit(&empty[s]);
                 }
-                if (alive) umma_commit(&tmem_full[buf]);
+                if (alive && kblocks > 0) umma_commit(&tmem_full[buf]);
             }
+        }
+    } else if (SHARED) {
+        // ---------------- sums of this share into the place of the stages (all of which the MMAs have read) ----------------
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * LDS + half * (BN / 2);
+        bool alive = kblocks == 0 || mbar_wait_bounded(&tmem_full[0], 0, p.status);
+        alive = __all_sync(0xffffffffu, alive);
+        tc_fence_after();
+#pragma unroll
+        for (int j = 0; j < BN / 2; j += 32) {
+            uint32_t r[32];
+            if (kblocks > 0) {
+                tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2) + j, r);
+                tmem_ld_wait();
+            } else {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) r[e] = 0;
+            }
+            if (alive)
+#pragma unroll
+                for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(row + j + e) = make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);
         }
     } else {
         // ---------------- epilogue warps ----------------
@@ -197,7 +239,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const Activation act = activation_of(p.c.act);
         int local = 0, tile_row0, tn;
         bool alive = true;
-        for (int tile = blockIdx.x; alive && decode_tile(p, tile, tile_row0, tn); tile += gridDim.x, ++local) {
+        for (int tile = first; alive && decode_tile(p, tile, tile_row0, tn); tile += stride, ++local) {
             const int buf = local & 1;
             alive = mbar_wait_bounded(&tmem_full[buf], (local >> 1) & 1, p.status);
             alive = __all_sync(0xffffffffu, alive);
@@ -260,6 +302,15 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
     }
 
+    if constexpr (SHARED) {
+        int row0, tn;
+        decode_tile(p, first, row0, tn);
+        __syncwarp();
+        cluster_sync_all();
+        finish_shares<BN, LDS, kThreads>(p.c, smem_u32(smem), p.split, share, tn, row0, BM, p.vec, [](int, int, float v) { return v; });
+        cluster_sync_all();                                // nobody leaves while a neighbour may still read its sums
+    }
+
     // common exit: all roles meet, then the allocating warp releases TMEM
     tc_fence_before();
     __syncthreads();
@@ -269,19 +320,21 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
 }
 
-template <int BN, bool RES>
+template <int BN, bool RES, bool SHARED>
 cudaError_t launch_kernel(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t st) {
     static bool done[64] = {};
     constexpr size_t smem = smem_for(BN);
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
-    const cudaError_t e = allow_smem(dense_tcgen05_kernel<BN, RES>, smem, done);
+    const cudaError_t e = allow_smem(dense_tcgen05_kernel<BN, RES, SHARED>, smem, done);
     if (e != cudaSuccess) return e;
     const int tiles = p.tiles_m * p.tiles_n;
-    return launch_dependent(dense_tcgen05_kernel<BN, RES>, dim3(tiles < kNumSm ? tiles : kNumSm), dim3(kThreads), smem, st, ma, mb, p);
+    if (SHARED) return launch_dependent_cluster(dense_tcgen05_kernel<BN, RES, SHARED>, dim3(tiles * p.split), p.split, dim3(kThreads), smem, st, ma, mb, p);
+    return launch_dependent(dense_tcgen05_kernel<BN, RES, SHARED>, dim3(tiles < kNumSm ? tiles : kNumSm), dim3(kThreads), smem, st, ma, mb, p);
 }
 template <int BN>
 cudaError_t launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t st) {
-    return p.c.residual ? launch_kernel<BN, true>(ma, mb, p, st) : launch_kernel<BN, false>(ma, mb, p, st);
+    if (p.split > 1) return launch_kernel<BN, false, true>(ma, mb, p, st);
+    return p.c.residual ? launch_kernel<BN, true, false>(ma, mb, p, st) : launch_kernel<BN, false, false>(ma, mb, p, st);
 }
 
 }  // namespace
@@ -299,16 +352,25 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     const int cols = c.pair_cols ? c.pair_cols : c.N;
     p.vec = (cols % 4 == 0) && (c.ldo % 4 == 0) && (reinterpret_cast<uintptr_t>(c.out_f32) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(c.out_b16) & 7) == 0 && (reinterpret_cast<uintptr_t>(c.residual) & 15) == 0;
-    // the widest tile that fills the SMs
-    int bn = c.N > 128 ? 256 : (c.N > 64 ? 128 : 64);
-    const long long tm = (c.M + BM - 1) / BM;
-    auto tiles = [&](int b) { return tm * ((c.N + b - 1) / b); };
-    auto fill = [&](int b) {
-        const long long t = tiles(b);
-        return static_cast<double>(t) / (static_cast<double>((t + kNumSm - 1) / kNumSm) * kNumSm);
-    };
-    if (bn == 256 && fill(128) > 1.15 * fill(256)) bn = 128;
-    if (bn == 128 && tiles(128) < 100 && c.N > 64) bn = 64;
+    // Tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
+    // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to
+    // measurements.  64 x 12288 x 4096: 64 tiles of 64 columns took 62 us, 32 of 128 in four shares 23; 512 x 6144 x 2048:
+    // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.
+    const long long tm = (c.M + BM - 1) / BM, kb = (c.K + BKE - 1) / BKE;
+    const int a_rows = c.M < 64 ? 64 : (c.M < BM ? static_cast<int>(c.M) : BM);
+    int bn = 64, split = 1;
+    double best = 0.0;
+    for (int b = 256; b >= 64; b /= 2) {
+        if (b > 64 && c.N <= b / 2) continue;
+        const long long tiles = tm * ((c.N + b - 1) / b);
+        for (int s = 1; s <= kMaxSplit; s *= 2) {
+            if (s > 1 && (kb < 4 * s || tiles * s > cluster_room(dense_tcgen05_kernel<256, false, true>, s, kThreads, smem_for(256)))) break;
+            const double blocks = static_cast<double>((tiles + kNumSm - 1) / kNumSm) * ((kb + s - 1) / s);
+            const double us = blocks * (0.12 + 0.95e-3 * (a_rows + b)) + (s > 1 ? 1.7 + 3.9e-4 * a_rows * b / s : 0.0);
+            if (best == 0.0 || us < best) { best = us; bn = b; split = s; }
+        }
+    }
+    p.split = split;
     p.tiles_m = static_cast<int>(tm);
     p.tiles_n = (c.N + bn - 1) / bn;
     CUtensorMap ma, mb;

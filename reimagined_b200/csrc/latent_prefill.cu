@@ -301,7 +301,7 @@ int launch_latent_expanded(const tbl_latent_mixer& m, const LatentParams& p, int
     int rc = launch_dense(TBL_BF16, kDenseTensor, k, st);
     if (rc != TBL_OK) return rc;
     DenseCall v{};
-    v.x = p.uv; v.w = gathered; v.ldx = p.R; v.ldw = p.cw; v.M = p.H * p.vd; v.K = p.R; v.N = n_seq * ctx; v.out_b16 = p.values; v.ldo = v.N;
+    v.x = p.uv; v.w = gathered; v.ldx = p.R; v.ldw = p.cw; v.M = p.H * p.vd; v.K = p.R; v.N = n_seq * ctx; v.out_b16 = p.values; v.ldo = v.N; v.w_computed = 1;
     rc = launch_dense(TBL_BF16, kDenseTensor, v, st);
     if (rc != TBL_OK) return rc;
     bf16* q = static_cast<bf16*>(p.qa);

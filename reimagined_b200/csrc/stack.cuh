@@ -107,6 +107,7 @@ struct DenseCall {
     const bf16* w;           // [N, K], ldw between rows (0: K)
     const float* bias;       // [N] or null
     int ldx, M, K, N, ldw;
+    int w_computed;          // w is what an earlier kernel of the step wrote (tensor-core route only): no load of it before the wait
     float* out_f32;          // exactly one of the two outputs
     bf16* out_b16;
     int ldo, act;            // act: TBL_ACT_* of a gated pair
@@ -127,6 +128,7 @@ bool dense_tensor_supported(const DenseCall& c);
 cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st);
 bool dense_split_supported(const DenseCall& c);
 cudaError_t launch_dense_split(const DenseCall& c, cudaStream_t st);
+static_assert(sizeof(DenseCall) == 128, "eight bytes more and the row-streaming kernel's launches take a tenth longer");
 
 // ---- stack_glue.cu ----------------------------------------------------------------------------------------------
 struct DepthNorm {

@@ -89,6 +89,28 @@ def test_dense_tall_tiles_and_the_residual_in_place(cuda, stack_lib):
     assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("m,k,n,ff", [(1, 512, 8, 8), (64, 1024, 130, 70), (65, 520, 2050, 1000), (128, 4104, 257, 97), (129, 8192, 64, 32),
+                                      (512, 3072, 1024, 1030), (700, 1032, 1026, 515)])
+def test_dense_shares_of_k(cuda, stack_lib, m, k, n, ff):
+    """Few tiles and a long K: the CTAs of a cluster share a tile's K (two or four shares, the last one short) and its rows."""
+    from reimagined_b200.stack import StackEngine
+    torch, rng = cuda, np.random.default_rng(m * k + n)
+    b = Buf(torch)
+    x = act(torch, rng.standard_normal((m, k)), 1)
+    w, gate, up = (torch.as_tensor(rng.standard_normal((r, k)) * k ** -0.5, dtype=torch.float32).bfloat16() for r in (n, ff, ff))
+    bias = rng.standard_normal(n)
+    out = torch.as_tensor(rng.standard_normal((m, n)), dtype=torch.float32).cuda()
+    want = out.double() + x.double() @ w.cuda().double().T + torch.as_tensor(bias).cuda()
+    assert stack_lib.tbl_dense_forward(C.byref(b.view(w, bias)), 1, TENSOR, x.data_ptr(), k, m, out.data_ptr(), out.data_ptr(), stream(torch)) == 0
+    assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-5          # as for whole tiles
+    h = torch.full((m, ff), float("nan"), device="cuda", dtype=torch.bfloat16)
+    paired = b.view(StackEngine._paired(None, gate, up))
+    assert stack_lib.tbl_gated_dense_forward(C.byref(paired), 1, TENSOR, x.data_ptr(), k, m, ff, h.data_ptr(), stream(torch)) == 0
+    gw, uw = (x.double() @ t.cuda().double().T for t in (gate, up))
+    assert_close(f64(h), (torch.nn.functional.silu(gw) * uw).cpu().numpy(), 4e-3)
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
 @pytest.mark.parametrize("m,k,ff", [(9, 512, 70), (1, 64, 32), (3, 40, 37), (4, 128, 200), (1, 1024, 3000), (150, 72, 100), (260, 136, 333)])
 def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
