@@ -22,9 +22,10 @@ __device__ __forceinline__ uint4 ld_stream(const bf16* p) {
 }
 
 // TA: 16-row weight tiles per warp (a gated layer: the gate tile and its up tile).  NB: blocks of 8 activation rows.
-template <int TA, int NB>
-__global__ void __launch_bounds__(32 * kWarps) dense_rows_kernel(const DenseCall c, const int wk) {
-    constexpr int U = TA == 1 ? 4 : 2;                     // steps of 32 in flight per batch of loads
+// U: steps of 32 per batch of loads, two of which are in flight.  CTAS: CTAs that an SM is to have room for (0: left to
+// the compiler).
+template <int TA, int NB, int U, int CTAS>
+__global__ void __launch_bounds__(32 * kWarps, CTAS) dense_rows_kernel(const DenseCall c, const int wk) {
     constexpr int LDP = NB * 8 + 1;
     extern __shared__ float part[];                        // [warps][TA * 16][LDP]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -117,18 +118,35 @@ __global__ void __launch_bounds__(32 * kWarps) dense_rows_kernel(const DenseCall
     }
 }
 
-template <int TA, int NB>
-cudaError_t launch(const DenseCall& c, cudaStream_t st) {
+template <int TA, int NB, int U, int CTAS>
+cudaError_t launch_u(const DenseCall& c, dim3 grid, int wk, cudaStream_t st) {
     static bool done[64] = {};
     const size_t smem = sizeof(float) * kWarps * TA * 16 * (NB * 8 + 1);
-    const cudaError_t e = allow_smem(dense_rows_kernel<TA, NB>, smem, done);
+    const cudaError_t e = allow_smem(dense_rows_kernel<TA, NB, U, CTAS>, smem, done);
     if (e != cudaSuccess) return e;
+    return launch_dependent(dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
+}
+
+template <int TA, int NB>
+cudaError_t launch(const DenseCall& c, cudaStream_t st) {
     const int batch = c.batch > 0 ? c.batch : 1;
     const int units = c.pair_cols ? ceil_div(c.pair_cols, 16) : ceil_div(c.N, 16 * TA);
     int wk = 1;
     while (wk < kWarps && static_cast<long long>(units) * batch * wk < 148 * 14 && c.K >= 256 * wk) wk *= 2;
-    return launch_dependent(dense_rows_kernel<TA, NB>, dim3(ceil_div(units, kWarps / wk), batch, ceil_div(c.M, NB * 8)), dim3(32 * kWarps), smem, st,
-                            c, wk);
+    const dim3 grid(ceil_div(units, kWarps / wk), batch, ceil_div(c.M, NB * 8));
+    const long long ctas = static_cast<long long>(grid.x) * batch * grid.z;
+    // The loads in flight against the CTAs that run at once (64 .. 102 and 190 registers): many CTAs want to be one wave --
+    // 2048 -> 10304 at one row is 322 of them, which took 12.4 us two to an SM with four steps a batch and take 8.7 three to an
+    // SM with two; 32000 rows 26 and 24 us four to an SM; 16 rows of a gated 4096 -> 12288 58 and 36 us.  So few that an
+    // SM has one keep more on its way: 6144 -> 2048 8.8 and 7.4 us with eight steps.
+    if constexpr (TA == 1 && NB <= 2) {
+        if (ctas > 3 * kNumSm && NB == 1) return launch_u<TA, NB, 2, NB == 1 ? 4 : 3>(c, grid, wk, st);
+        if (ctas > 2 * kNumSm) return launch_u<TA, NB, 2, 3>(c, grid, wk, st);
+        if (NB == 1 && ctas <= kNumSm && c.K >= 512 * wk) return launch_u<TA, NB, NB == 1 ? 8 : 4, NB == 1 ? 1 : 0>(c, grid, wk, st);
+    }
+    if constexpr (TA == 2 && NB == 2)
+        if (ctas > 2 * kNumSm) return launch_u<TA, NB, 1, 3>(c, grid, wk, st);
+    return launch_u<TA, NB, TA == 1 ? 4 : 2, 0>(c, grid, wk, st);
 }
 
 template <int TA>

@@ -111,6 +111,19 @@ def test_dense_shares_of_k(cuda, stack_lib, m, k, n, ff):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 264, 148 * 16), (1, 5000, 148 * 16 + 1), (8, 512, 1200), (16, 520, 148 * 64), (9, 520, 148 * 64 + 9), (3, 264, 32000), (16, 2056, 37888)])
+def test_dense_rows_by_the_number_of_blocks(cuda, stack_lib, m, k, n):
+    """Row-streaming kernel: one block to an SM and a long K, two, three, four blocks to an SM, and one more than a wave."""
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, w = torch.randn(m, k).bfloat16().cuda(), torch.randn(n, k).bfloat16()
+    out = torch.full((m, n), float("nan"), device="cuda")
+    assert stack_lib.tbl_dense_forward(C.byref(b.view(w)), 1, ROWS, x.data_ptr(), k, m, None, out.data_ptr(), stream(torch)) == 0
+    want = x.double() @ w.cuda().double().T
+    assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-5
+
+
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
 @pytest.mark.parametrize("m,k,ff", [(9, 512, 70), (1, 64, 32), (3, 40, 37), (4, 128, 200), (1, 1024, 3000), (150, 72, 100), (260, 136, 333)])
 def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
