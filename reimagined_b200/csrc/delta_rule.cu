@@ -5,9 +5,10 @@
 // columns are spread over threads and CTAs and only the dot products over the keys cross lanes: eight or sixteen lanes
 // share a column, each holding its groups of four keys in registers, and the arithmetic runs on packed fp32 pairs.
 //
-//   delta_scan_kernel   a sequence of tokens, two per round: a CTA owns 32 columns of a head.  Eight producer warps turn
-//                       the raw projections of the next sixteen tokens into records in shared memory while four
-//                       consumer warps walk the current ones with the state in registers.
+//   delta_records_kernel  turns the raw projections of two tokens into a record: everything a round of the scan multiplies
+//                       with, once per head instead of once per block of columns.
+//   delta_scan_kernel   a sequence of tokens, two per round: a CTA owns 8, 16 or 32 columns of a head.  A producer brings the
+//                       records by bulk copies, four warps walk them with the state in registers.
 //   delta_step_kernel   one token: a CTA per head also computes the low-rank decay product, the head norm and the gate.
 #include "stack.cuh"
 
@@ -30,8 +31,6 @@ __device__ __forceinline__ float sum8lanes(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 4);
     return v;
 }
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // Four keys of one column (key index c .. c+3, clipped at dim): state <-> registers.
 __device__ __forceinline__ ulonglong2 load_state4(const float* col, int c, int dim) {
@@ -65,14 +64,17 @@ struct DeltaParams {
     float* states;           // [slots][heads][dim][dim]
     const int32_t* slots;
     float* o;                // [rows][heads*dim] raw readouts (scan kernel)
+    float* records;          // [seq][head][round][record] (scan kernel)
+    int* status;
     void* out;
     int ld, heads, dim, rank, n_tok;
+    int seq0, tok0, some;    // scan kernel: first sequence and token of this launch, and how many tokens of each
     float rate, key_eps, eps;
 };
 
-constexpr int kScanCols = 32;          // value columns per CTA
-constexpr int kProducers = 8;          // producer warps: enough tokens in flight to cover the loads' latency
-constexpr int kScanThreads = 32 * (4 + kProducers);
+constexpr int kScanLanes = 8;          // groups of sixteen lanes in the consumer warps; each has NC value columns
+constexpr int kScanThreads = 32 * 5;   // four consumer warps, one producer
+constexpr int kStageRounds = 4;        // rounds per bulk copy
 
 // The scan takes two tokens per round.  With w, u, q = a * u, k, r, v of the two tokens (0 and 1) and the state S before
 // them, everything the round needs from S are four dot products per column, taken together:
@@ -84,13 +86,18 @@ constexpr int kScanThreads = 32 * (4 + kProducers);
 //     S  <- (w0 w1) S + (w1 k0) v0 - (w1 q0) d0 + k1 v1 - q1 d1
 // An odd last token is followed by one that changes nothing (w = 1, the others 0).
 template <int DKP>
-struct ScanShape {
-    static constexpr int kPairs = kProducers;                          // rounds per buffer: one per producer warp
+struct Record {
     static constexpr int kScalars = 9 * DKP;                           // 12 products of the tokens with each other
-    static constexpr int kValues = kScalars + 16;                      // v of both tokens, this CTA's columns
-    static constexpr int kRecord = kValues + 2 * kScanCols;            // floats per round
-    static constexpr size_t kSmem = sizeof(float) * 2 * kPairs * kRecord;
+    static constexpr int kValues = kScalars + 16;                      // v of both tokens
+    static constexpr int kFloats = kValues + 2 * DKP;
+    static constexpr int kStageBytes = 4 * kStageRounds * kFloats;
+    static constexpr int kStages = DKP == 256 ? 4 : 6;                 // bulk copies on their way or in use
 };
+// Most records of a head at a time: longer sequences are scanned in pieces, more sequences in groups, so that the records
+// between the two kernels stay in L2 (16 heads of 128: 93 MB).
+constexpr int kMaxRounds = 1024;
+inline int padded_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : 256); }
+inline size_t record_floats(int dim) { return 11 * static_cast<size_t>(padded_dim(dim)) + 16; }
 
 __device__ __forceinline__ float pick4(const float (&v)[4], int n) {
     const float a = n & 1 ? v[1] : v[0], b = n & 1 ? v[3] : v[2];
@@ -101,209 +108,244 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf
 // (a division good to two units in the last place)
 __device__ __forceinline__ float sigmoid_near(float z) { return __fdividef(1.0f, 1.0f + expf(-z)); }
 
+// One warp per record; lane l has channels 4l .. 4l + 3 (+ 128).
 template <int DKP>
-__global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaParams p) {
-    using Shape = ScanShape<DKP>;
-    constexpr int PAIRS = Shape::kPairs, REC = Shape::kRecord;
+__global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p, const int n_seq) {
+    using R = Record<DKP>;
+    constexpr int NI = (DKP + 127) / 128;      // groups of four channels per lane
+    const int lane = threadIdx.x & 31, dim = p.dim, HD = p.heads * dim, rounds = (p.some + 1) / 2;
+    // neighbouring warps take neighbouring heads of the same tokens: their rows are one piece of memory
+    const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    const int head = static_cast<int>(unit % p.heads);
+    const size_t at = unit / p.heads;
+    const int seq = static_cast<int>(at / rounds), t0 = 2 * static_cast<int>(at - static_cast<size_t>(seq) * rounds);
+    pdl_launch_dependents();
+    if (seq >= n_seq) return;
+    const bool vec = ((dim | p.ld) & 3) == 0;          // every row and head starts on 16 bytes
+    auto load4 = [&](const float* base, int c, bool live) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!live || c >= dim) return v;
+        if (vec) return *reinterpret_cast<const float4*>(base + c);
+        v.x = base[c];
+        if (c + 1 < dim) v.y = base[c + 1];
+        if (c + 2 < dim) v.z = base[c + 2];
+        if (c + 3 < dim) v.w = base[c + 3];
+        return v;
+    };
+    pdl_wait();
+    const bool second = t0 + 1 < p.some;
+    float4 r[2][NI], k[2][NI], u[2][NI], q[2][NI], w[2][NI], v[2][NI];
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const bool live = s == 0 || second;
+        const size_t row_at = static_cast<size_t>(p.seq0 + seq) * p.n_tok + p.tok0 + t0 + (live ? s : 0);
+        const float* row = p.proj + row_at * p.ld + head * dim;
+        const float* zr = p.z + row_at * HD + head * dim;
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int c = 4 * lane + 128 * i;
+            r[s][i] = load4(row, c, live);
+            k[s][i] = load4(row + HD, c, live);
+            v[s][i] = load4(row + 2 * HD, c, live);
+            q[s][i] = load4(row + 4 * HD, c, live);
+            w[s][i] = load4(zr, c, live);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        s0 = dot4(k[0][i], k[0][i], s0);
+        s1 = dot4(k[1][i], k[1][i], s1);
+    }
+    const float i0 = 1.0f / sqrtf(warp_sum(s0) + p.key_eps), i1 = 1.0f / sqrtf(warp_sum(s1) + p.key_eps);
+    auto decay = [&](float z) { return expf(-p.rate * sigmoid_near(z)); };
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const float n = s ? i1 : i0;
+            const float4 w0 = load4(p.w0 + head * dim, 4 * lane + 128 * i, true), a = q[s][i], z = w[s][i];
+            u[s][i] = mul4(k[s][i], make_float4(n, n, n, n));
+            q[s][i] = mul4(make_float4(sigmoid_near(a.x), sigmoid_near(a.y), sigmoid_near(a.z), sigmoid_near(a.w)), u[s][i]);
+            w[s][i] = make_float4(decay(z.x + w0.x), decay(z.y + w0.y), decay(z.z + w0.z), decay(z.w + w0.w));
+            if (s == 1 && !second) w[s][i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        }
+    float* rec = p.records + ((static_cast<size_t>(seq) * p.heads + head) * rounds + t0 / 2) * R::kFloats;
+    float m[8] = {};
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int c = 4 * lane + 128 * i;
+        const float4 k0w = mul4(w[1][i], k[0][i]), q0w = mul4(w[1][i], q[0][i]), ww = mul4(w[0][i], w[1][i]);
+        m[0] = dot4(r[0][i], k[0][i], m[0]); m[1] = dot4(r[0][i], q[0][i], m[1]);
+        m[2] = dot4(r[1][i], k0w, m[2]);     m[3] = dot4(r[1][i], q0w, m[3]);
+        m[4] = dot4(r[1][i], k[1][i], m[4]); m[5] = dot4(r[1][i], q[1][i], m[5]);
+        m[6] = dot4(u[1][i], k[0][i], m[6]); m[7] = dot4(u[1][i], q[0][i], m[7]);
+        if (c >= DKP) continue;
+        *reinterpret_cast<float4*>(rec + c) = u[0][i];
+        *reinterpret_cast<float4*>(rec + DKP + c) = mul4(u[1][i], w[0][i]);
+        *reinterpret_cast<float4*>(rec + 2 * DKP + c) = mul4(r[0][i], w[0][i]);
+        *reinterpret_cast<float4*>(rec + 3 * DKP + c) = mul4(r[1][i], ww);
+        *reinterpret_cast<float4*>(rec + 4 * DKP + c) = ww;
+        *reinterpret_cast<float4*>(rec + 5 * DKP + c) = k0w;
+        *reinterpret_cast<float4*>(rec + 6 * DKP + c) = q0w;
+        *reinterpret_cast<float4*>(rec + 7 * DKP + c) = k[1][i];
+        *reinterpret_cast<float4*>(rec + 8 * DKP + c) = q[1][i];
+        *reinterpret_cast<float4*>(rec + R::kValues + c) = v[0][i];
+        *reinterpret_cast<float4*>(rec + R::kValues + DKP + c) = v[1][i];
+    }
+    // the eight products over the lanes: after three exchanges a lane holds one of them, number lane / 4
+    float m4[4], m2[2];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        m4[e] = (lane & 16 ? m[e + 4] : m[e]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? m[e] : m[e + 4], 16);
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        m2[e] = (lane & 8 ? m4[e + 2] : m4[e]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? m4[e] : m4[e + 2], 8);
+    float m1 = (lane & 4 ? m2[1] : m2[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? m2[0] : m2[1], 4);
+    m1 += __shfl_xor_sync(0xffffffffu, m1, 2);
+    m1 += __shfl_xor_sync(0xffffffffu, m1, 1);
+    // token 0: factors of v0, d0, v1, d1; token 1: the same; then those of d1 (and nothing)
+    float* sc = rec + R::kScalars;
+    if ((lane & 3) == 0) {
+        const int e = lane >> 2;
+        sc[e < 2 ? e : e + 2] = m1;
+        if (e < 2) sc[2 + e] = 0.0f;
+    }
+    if (lane < 6) sc[10 + lane] = 0.0f;
+}
+
+// What bounds it is a round's chain from the state through the dot products and their sums over sixteen lanes back to the
+// state, so the columns are spread over as many SMs as there are.  Every wait is bounded.
+template <int DKP, int NC>
+__global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaParams p, const int stages) {
+    using R = Record<DKP>;
+    constexpr int COLS = kScanLanes * NC;      // value columns per CTA
     constexpr int G = DKP / 64;                // groups of four keys per consumer lane: 4 (l + 16 g), l = lane % 16
-    constexpr int NI = (DKP + 127) / 128;      // groups of four channels per producer lane
-    extern __shared__ __align__(16) float sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int head = blockIdx.y, seq = blockIdx.z, j0 = blockIdx.x * kScanCols;
+    extern __shared__ __align__(128) float sm[];
+    __shared__ __align__(8) uint64_t full[R::kStages], empty[R::kStages];
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int head = blockIdx.y, seq = blockIdx.z, j0 = blockIdx.x * COLS;
     const int dim = p.dim, HD = p.heads * dim;
-    const int chunks = (p.n_tok + 2 * PAIRS - 1) / (2 * PAIRS);
-    const size_t row0 = static_cast<size_t>(seq) * p.n_tok;
+    const int rounds = (p.some + 1) / 2, chunks = (rounds + kStageRounds - 1) / kStageRounds;
+    const size_t row0 = static_cast<size_t>(p.seq0 + seq) * p.n_tok + p.tok0;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        fence_mbar_init();
+        fence_proxy_async();
+    }
+    __syncthreads();
     pdl_launch_dependents();
     pdl_wait();
-    if (warp >= 4) {
-        // ---- producers: warp w takes round w of every buffer; lane l channels 4l .. 4l + 3 (+ 128) ----
-        const int pw = warp - 4;
-        const bool vec = ((dim | p.ld) & 3) == 0;      // every row and head starts on 16 bytes
-        auto load4 = [&](const float* base, int c, bool live) {
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (!live || c >= dim) return v;
-            if (vec) return *reinterpret_cast<const float4*>(base + c);
-            v.x = base[c];
-            if (c + 1 < dim) v.y = base[c + 1];
-            if (c + 2 < dim) v.z = base[c + 2];
-            if (c + 3 < dim) v.w = base[c + 3];
-            return v;
-        };
-        float4 w0[NI], nr[2][NI], nk[2][NI], na[2][NI], nz[2][NI];
-        float nv[2];
-#pragma unroll
-        for (int i = 0; i < NI; ++i) w0[i] = load4(p.w0 + head * dim, 4 * lane + 128 * i, true);
-        auto fetch = [&](int t0) {
-#pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const bool live = t0 + s < p.n_tok;
-                const size_t at = row0 + (live ? t0 + s : 0);
-                const float* row = p.proj + at * p.ld + head * dim;
-                const float* zr = p.z + at * HD + head * dim;
-#pragma unroll
-                for (int i = 0; i < NI; ++i) {
-                    const int c = 4 * lane + 128 * i;
-                    nr[s][i] = load4(row, c, live);
-                    nk[s][i] = load4(row + HD, c, live);
-                    na[s][i] = load4(row + 4 * HD, c, live);
-                    nz[s][i] = load4(zr, c, live);
-                }
-                nv[s] = live && j0 + lane < dim ? row[2 * HD + j0 + lane] : 0.0f;
+    if (warp == 4) {
+        if (lane == 0) {
+            const float* src = p.records + (static_cast<size_t>(seq) * p.heads + head) * rounds * R::kFloats;
+            int ch = 0;
+            bool alive = true;
+            for (; ch < chunks; ++ch) {
+                const int s = ch % stages, n = min(kStageRounds, rounds - ch * kStageRounds);
+                if (ch >= stages) alive = mbar_wait_bounded(&empty[s], ((ch / stages) - 1) & 1, p.status);
+                if (!alive) break;
+                mbar_arrive_expect_tx(&full[s], 4 * n * R::kFloats);
+                bulk_g2s(sm + s * kStageRounds * R::kFloats, src + static_cast<size_t>(ch) * kStageRounds * R::kFloats, 4 * n * R::kFloats, &full[s]);
             }
-        };
-        fetch(2 * pw);
-        for (int ch = 0; ch < chunks; ++ch) {
-            const int b = ch & 1, t0 = 2 * (ch * PAIRS + pw);
-            if (ch >= 2) bar_sync(3 + b, kScanThreads);
-            if (t0 < p.n_tok) {
-                float4 r[2][NI], k[2][NI], u[2][NI], q[2][NI], w[2][NI];
-                const float v0 = nv[0], v1 = nv[1];
-                float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll
-                for (int i = 0; i < NI; ++i) {
-                    s0 = dot4(nk[0][i], nk[0][i], s0);
-                    s1 = dot4(nk[1][i], nk[1][i], s1);
-                }
-                const float i0 = 1.0f / sqrtf(warp_sum(s0) + p.key_eps), i1 = 1.0f / sqrtf(warp_sum(s1) + p.key_eps);
-                const bool second = t0 + 1 < p.n_tok;
-                auto decay = [&](float z) { return expf(-p.rate * sigmoid_near(z)); };
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-#pragma unroll
-                    for (int i = 0; i < NI; ++i) {
-                        const float n = s ? i1 : i0;
-                        r[s][i] = nr[s][i];
-                        k[s][i] = nk[s][i];
-                        u[s][i] = mul4(k[s][i], make_float4(n, n, n, n));
-                        q[s][i] = mul4(make_float4(sigmoid_near(na[s][i].x), sigmoid_near(na[s][i].y), sigmoid_near(na[s][i].z), sigmoid_near(na[s][i].w)), u[s][i]);
-                        w[s][i] = make_float4(decay(nz[s][i].x + w0[i].x), decay(nz[s][i].y + w0[i].y), decay(nz[s][i].z + w0[i].z), decay(nz[s][i].w + w0[i].w));
-                        if (s == 1 && !second) w[s][i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-                    }
-                fetch(t0 + 2 * PAIRS);
-                float* rec = sm + static_cast<size_t>(b * PAIRS + pw) * REC;
-                float m[8] = {};
-#pragma unroll
-                for (int i = 0; i < NI; ++i) {
-                    const int c = 4 * lane + 128 * i;
-                    const float4 k0w = mul4(w[1][i], k[0][i]), q0w = mul4(w[1][i], q[0][i]), ww = mul4(w[0][i], w[1][i]);
-                    m[0] = dot4(r[0][i], k[0][i], m[0]); m[1] = dot4(r[0][i], q[0][i], m[1]);
-                    m[2] = dot4(r[1][i], k0w, m[2]);     m[3] = dot4(r[1][i], q0w, m[3]);
-                    m[4] = dot4(r[1][i], k[1][i], m[4]); m[5] = dot4(r[1][i], q[1][i], m[5]);
-                    m[6] = dot4(u[1][i], k[0][i], m[6]); m[7] = dot4(u[1][i], q[0][i], m[7]);
-                    if (c >= DKP) continue;
-                    *reinterpret_cast<float4*>(rec + c) = u[0][i];
-                    *reinterpret_cast<float4*>(rec + DKP + c) = mul4(u[1][i], w[0][i]);
-                    *reinterpret_cast<float4*>(rec + 2 * DKP + c) = mul4(r[0][i], w[0][i]);
-                    *reinterpret_cast<float4*>(rec + 3 * DKP + c) = mul4(r[1][i], ww);
-                    *reinterpret_cast<float4*>(rec + 4 * DKP + c) = ww;
-                    *reinterpret_cast<float4*>(rec + 5 * DKP + c) = k0w;
-                    *reinterpret_cast<float4*>(rec + 6 * DKP + c) = q0w;
-                    *reinterpret_cast<float4*>(rec + 7 * DKP + c) = k[1][i];
-                    *reinterpret_cast<float4*>(rec + 8 * DKP + c) = q[1][i];
-                }
-                // the eight products over the lanes: after three exchanges a lane holds one of them, number lane / 4
-                float m4[4], m2[2];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    m4[e] = (lane & 16 ? m[e + 4] : m[e]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? m[e] : m[e + 4], 16);
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    m2[e] = (lane & 8 ? m4[e + 2] : m4[e]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? m4[e] : m4[e + 2], 8);
-                float m1 = (lane & 4 ? m2[1] : m2[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? m2[0] : m2[1], 4);
-                m1 += __shfl_xor_sync(0xffffffffu, m1, 2);
-                m1 += __shfl_xor_sync(0xffffffffu, m1, 1);
-                // token 0: factors of v0, d0, v1, d1; token 1: the same; then those of d1
-                float* sc = rec + Shape::kScalars;
-                if ((lane & 3) == 0) {
-                    const int e = lane >> 2;
-                    sc[e < 2 ? e : e + 2] = m1;
-                    if (e < 2) sc[2 + e] = 0.0f;
-                }
-                rec[Shape::kValues + lane] = v0;
-                rec[Shape::kValues + kScanCols + lane] = v1;
-            }
-            __threadfence_block();
-            bar_arrive(1 + b, kScanThreads);
+            if (!alive)                                    // nobody else may be waiting for the copies in flight
+                for (int j = max(0, ch - stages); j < ch; ++j) mbar_wait_bounded(&full[j % stages], (j / stages) & 1, p.status);
         }
         return;
     }
-    // ---- consumers: sixteen lanes share the keys of four columns ----
-    const int l = lane & 15, base = lane & 16, cl = warp * 8 + (base >> 2);       // first of this lane's columns within the CTA
-    float* st = p.states + (static_cast<size_t>(p.slots[seq]) * p.heads + head) * dim * dim;
-    ulonglong2 S[4][G];
+    // ---- consumers: sixteen lanes share the keys of NC columns ----
+    const int l = lane & 15, base = lane & 16, cl = (2 * warp + (base >> 4)) * NC;       // first of this lane's columns within the CTA
+    float* st = p.states + (static_cast<size_t>(p.slots[p.seq0 + seq]) * p.heads + head) * dim * dim;
+    ulonglong2 S[NC][G];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < NC; ++n)
 #pragma unroll
         for (int g = 0; g < G; ++g)
             S[n][g] = j0 + cl + n < dim ? load_state4(st + static_cast<size_t>(j0 + cl + n) * dim, 4 * (l + 16 * g), dim) : make_ulonglong2(0, 0);
-    // after the sums over the lanes, lane l holds dot product l / 4 of column l % 4: lanes 8 .. 15 finish the two readouts
-    const int mine = l & 3, token = (l >> 2) & 1;
-    const bool writes = l >= 8 && j0 + cl + mine < dim;
+    // after the sums over the lanes, lane l holds dot product l / 4 of column l % 4 * NC / 4: lanes 8 .. 15 finish the two readouts
+    constexpr int STEP = 4 / NC;                           // lanes that hold the same sum
+    const int mine = (l & 3) / STEP, token = (l >> 2) & 1;
+    const bool writes = l >= 8 && l % STEP == 0 && j0 + cl + mine < dim;
     float* o = p.o + (row0 + token) * HD + head * dim + j0 + cl + mine;
+    auto pick = [&](const float (&v)[NC]) {
+        if constexpr (NC == 4) return pick4(v, mine);
+        else if constexpr (NC == 2) return mine ? v[1] : v[0];
+        else return v[0];
+    };
     for (int ch = 0; ch < chunks; ++ch) {
-        const int b = ch & 1;
-        bar_sync(1 + b, kScanThreads);
-        const int t0 = 2 * ch * PAIRS, rounds = min(PAIRS, (p.n_tok - t0 + 1) / 2);
+        const int b = ch % stages;
+        const bool alive = mbar_wait_bounded(&full[b], (ch / stages) & 1, p.status);
+        if (!__all_sync(0xffffffffu, alive)) break;
+        const int t0 = 2 * ch * kStageRounds, n_rounds = min(kStageRounds, rounds - ch * kStageRounds);
 #pragma unroll 1
-        for (int i = 0; i < rounds; ++i) {
-            const float* rec = sm + static_cast<size_t>(b * PAIRS + i) * REC;
+        for (int i = 0; i < n_rounds; ++i) {
+            const float* rec = sm + static_cast<size_t>(b * kStageRounds + i) * R::kFloats;
             const ulonglong2* q = reinterpret_cast<const ulonglong2*>(rec) + l;
             constexpr int V = DKP / 4;                     // 16-byte units per vector
-            float x[4][4];
+            float x[4][NC];
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
                 ulonglong2 c[G];
 #pragma unroll
                 for (int g = 0; g < G; ++g) c[g] = q[d * V + 16 * g];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
+                for (int n = 0; n < NC; ++n) {
                     pair2 a = mul2(c[0].x, S[n][0].x), e = mul2(c[0].y, S[n][0].y);
 #pragma unroll
                     for (int g = 1; g < G; ++g) { a = fma2(c[g].x, S[n][g].x, a); e = fma2(c[g].y, S[n][g].y, e); }
                     x[d][n] = sum2(add2(a, e));
                 }
             }
-            const float4 va = *reinterpret_cast<const float4*>(rec + Shape::kValues + cl), vb = *reinterpret_cast<const float4*>(rec + Shape::kValues + kScanCols + cl);
-            const float4 f = *reinterpret_cast<const float4*>(rec + Shape::kScalars + 4 * token);
-            const float2 fd = *reinterpret_cast<const float2*>(rec + Shape::kScalars + 8);
-            float y[2][4], z[4], h[2], r;
+            float v0[NC], v1[NC];
+#pragma unroll
+            for (int n = 0; n < NC; ++n) { v0[n] = rec[R::kValues + min(j0 + cl + n, DKP - 1)]; v1[n] = rec[R::kValues + DKP + min(j0 + cl + n, DKP - 1)]; }
+            const float4 f = *reinterpret_cast<const float4*>(rec + R::kScalars + 4 * token);
+            const float2 fd = *reinterpret_cast<const float2*>(rec + R::kScalars + 8);
+            float y[2][NC], z[NC], r;
 #pragma unroll
             for (int d = 0; d < 2; ++d)
 #pragma unroll
-                for (int n = 0; n < 4; ++n) y[d][n] = (l & 8 ? x[d + 2][n] : x[d][n]) + __shfl_xor_sync(0xffffffffu, l & 8 ? x[d][n] : x[d + 2][n], 8);
+                for (int n = 0; n < NC; ++n) y[d][n] = (l & 8 ? x[d + 2][n] : x[d][n]) + __shfl_xor_sync(0xffffffffu, l & 8 ? x[d][n] : x[d + 2][n], 8);
 #pragma unroll
-            for (int n = 0; n < 4; ++n) z[n] = (l & 4 ? y[1][n] : y[0][n]) + __shfl_xor_sync(0xffffffffu, l & 4 ? y[0][n] : y[1][n], 4);
+            for (int n = 0; n < NC; ++n) z[n] = (l & 4 ? y[1][n] : y[0][n]) + __shfl_xor_sync(0xffffffffu, l & 4 ? y[0][n] : y[1][n], 4);
+            if constexpr (NC == 4) {
+                float h[2];
 #pragma unroll
-            for (int n = 0; n < 2; ++n) h[n] = (l & 2 ? z[n + 2] : z[n]) + __shfl_xor_sync(0xffffffffu, l & 2 ? z[n] : z[n + 2], 2);
-            r = (l & 1 ? h[1] : h[0]) + __shfl_xor_sync(0xffffffffu, l & 1 ? h[0] : h[1], 1);
-            float d0[4], d1[4];
-            const float v0[4] = {va.x, va.y, va.z, va.w}, v1[4] = {vb.x, vb.y, vb.z, vb.w};
+                for (int n = 0; n < 2; ++n) h[n] = (l & 2 ? z[n + 2] : z[n]) + __shfl_xor_sync(0xffffffffu, l & 2 ? z[n] : z[n + 2], 2);
+                r = (l & 1 ? h[1] : h[0]) + __shfl_xor_sync(0xffffffffu, l & 1 ? h[0] : h[1], 1);
+            } else {
+                if constexpr (NC == 2) r = (l & 2 ? z[1] : z[0]) + __shfl_xor_sync(0xffffffffu, l & 2 ? z[0] : z[1], 2);
+                else r = z[0] + __shfl_xor_sync(0xffffffffu, z[0], 2);
+                r += __shfl_xor_sync(0xffffffffu, r, 1);
+            }
+            float d0[NC], d1[NC];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                d0[n] = __shfl_sync(0xffffffffu, r, base + n);
-                d1[n] = __shfl_sync(0xffffffffu, r, base + 4 + n);
+            for (int n = 0; n < NC; ++n) {
+                d0[n] = __shfl_sync(0xffffffffu, r, base + n * STEP);
+                d1[n] = __shfl_sync(0xffffffffu, r, base + 4 + n * STEP);
             }
 #pragma unroll
-            for (int n = 0; n < 4; ++n) d1[n] = fmaf(fd.x, v0[n], fmaf(-fd.y, d0[n], d1[n]));
-            pair2 p0[4], p1[4], m0[4], m1[4];
+            for (int n = 0; n < NC; ++n) d1[n] = fmaf(fd.x, v0[n], fmaf(-fd.y, d0[n], d1[n]));
+            pair2 p0[NC], p1[NC], m0[NC], m1[NC];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) { p0[n] = dup2(v0[n]); p1[n] = dup2(v1[n]); m0[n] = dup2(-d0[n]); m1[n] = dup2(-d1[n]); }
+            for (int n = 0; n < NC; ++n) { p0[n] = dup2(v0[n]); p1[n] = dup2(v1[n]); m0[n] = dup2(-d0[n]); m1[n] = dup2(-d1[n]); }
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 const ulonglong2 w = q[4 * V + 16 * g], k0 = q[5 * V + 16 * g], q0 = q[6 * V + 16 * g], k1 = q[7 * V + 16 * g], q1 = q[8 * V + 16 * g];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
+                for (int n = 0; n < NC; ++n) {
                     S[n][g].x = fma2(q1.x, m1[n], fma2(k1.x, p1[n], fma2(q0.x, m0[n], fma2(k0.x, p0[n], mul2(w.x, S[n][g].x)))));
                     S[n][g].y = fma2(q1.y, m1[n], fma2(k1.y, p1[n], fma2(q0.y, m0[n], fma2(k0.y, p0[n], mul2(w.y, S[n][g].y)))));
                 }
             }
-            const float out = fmaf(f.x, pick4(v0, mine), fmaf(-f.y, pick4(d0, mine), fmaf(f.z, pick4(v1, mine), fmaf(-f.w, pick4(d1, mine), r))));
-            if (writes && t0 + 2 * i + token < p.n_tok) o[static_cast<size_t>(t0 + 2 * i) * HD] = out;
+            const float out = fmaf(f.x, pick(v0), fmaf(-f.y, pick(d0), fmaf(f.z, pick(v1), fmaf(-f.w, pick(d1), r))));
+            if (writes && t0 + 2 * i + token < p.some) o[static_cast<size_t>(t0 + 2 * i) * HD] = out;
         }
-        if (ch + 2 < chunks) bar_arrive(3 + b, kScanThreads);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[b]);
     }
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < NC; ++n)
 #pragma unroll
         for (int g = 0; g < G; ++g)
             if (j0 + cl + n < dim) store_state4(st + static_cast<size_t>(j0 + cl + n) * dim, 4 * (l + 16 * g), dim, S[n][g]);
@@ -492,7 +534,7 @@ cudaError_t launch_step_d(const DeltaParams& p, dim3 grid, cudaStream_t st) {
 }
 
 struct Workspace {
-    float *z, *o;
+    float *z, *o, *records;
     void* th;
     size_t bytes;
 };
@@ -504,6 +546,8 @@ Workspace carve(const tbl_delta_mixer& m, int precision, size_t rows, void* base
     w.z = reinterpret_cast<float*>(take(sizeof(float) * rows * HD));
     w.o = reinterpret_cast<float*>(take(sizeof(float) * rows * HD));
     w.th = take(e * rows * round_up(m.rank, 8));
+    // (up to a round per row: a sequence of an odd number of tokens has half a round more)
+    w.records = reinterpret_cast<float*>(take(sizeof(float) * record_floats(m.dim) * m.heads * (rows < kMaxRounds ? rows : kMaxRounds)));
     return w;
 }
 
@@ -525,14 +569,28 @@ int launch_step(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
     return e == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 
+template <int DKP, int NC>
+int launch_scan_n(const DeltaParams& p, int n_seq, cudaStream_t st) {
+    static bool done[64] = {};
+    using R = Record<DKP>;
+    const int chunks = ceil_div((p.some + 1) / 2, kStageRounds), stages = chunks < R::kStages ? chunks : R::kStages;
+    if (allow_smem(delta_scan_kernel<DKP, NC>, static_cast<size_t>(R::kStages) * R::kStageBytes, done) != cudaSuccess) return TBL_ERR_CUDA;
+    const dim3 grid(ceil_div(p.dim, kScanLanes * NC), p.heads, n_seq);
+    if (p.heads > 65535 || n_seq > 65535) return TBL_ERR_SHAPE;
+    const long long units = static_cast<long long>(n_seq) * p.heads * ((p.some + 1) / 2);
+    if (launch_dependent(delta_records_kernel<DKP>, dim3(ceil_div(units, 8)), dim3(256), 0, st, p, n_seq) != cudaSuccess) return TBL_ERR_CUDA;
+    return launch_dependent(delta_scan_kernel<DKP, NC>, grid, dim3(kScanThreads), static_cast<size_t>(stages) * R::kStageBytes, st, p, stages) == cudaSuccess
+               ? TBL_OK : TBL_ERR_CUDA;
+}
+
 template <int DKP>
 int launch_scan_d(const DeltaParams& p, int n_seq, cudaStream_t st) {
-    static bool done[64] = {};
-    if (allow_smem(delta_scan_kernel<DKP>, ScanShape<DKP>::kSmem, done) != cudaSuccess) return TBL_ERR_CUDA;
-    const dim3 grid(ceil_div(p.dim, kScanCols), p.heads, n_seq);
-    if (p.heads > 65535 || n_seq > 65535) return TBL_ERR_SHAPE;
-    return launch_dependent(delta_scan_kernel<DKP>, grid, dim3(kScanThreads), ScanShape<DKP>::kSmem, st, p) == cudaSuccess ? TBL_OK
-                                                                                                                      : TBL_ERR_CUDA;
+    auto ctas = [&](int cols) { return static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq; };
+#ifdef SCANNC
+    return launch_scan_n<DKP, SCANNC>(p, n_seq, st);
+#endif
+    if (ctas(32) >= 100) return launch_scan_n<DKP, 4>(p, n_seq, st);
+    return ctas(16) >= 100 ? launch_scan_n<DKP, 2>(p, n_seq, st) : launch_scan_n<DKP, 1>(p, n_seq, st);
 }
 
 template <typename T>
@@ -543,10 +601,20 @@ int launch_scan(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
     int rc = decay_products<T>(m, p, precision, rows, static_cast<T*>(w.th), w.z, st);
     if (rc != TBL_OK) return rc;
     p.z = w.z;
-    if (p.dim <= 64) rc = launch_scan_d<64>(p, n_seq, st);
-    else if (p.dim <= 128) rc = launch_scan_d<128>(p, n_seq, st);
-    else rc = launch_scan_d<256>(p, n_seq, st);
-    if (rc != TBL_OK) return rc;
+    p.records = w.records;
+    p.status = device_status_ptr();
+    if (!p.status) return TBL_ERR_CUDA;
+    const int piece = p.n_tok < 2 * kMaxRounds ? p.n_tok : 2 * kMaxRounds, group = kMaxRounds / ((piece + 1) / 2);
+    for (p.seq0 = 0; p.seq0 < n_seq; p.seq0 += group) {
+        const int n = n_seq - p.seq0 < group ? n_seq - p.seq0 : group;
+        for (p.tok0 = 0; p.tok0 < p.n_tok; p.tok0 += piece) {
+            p.some = p.n_tok - p.tok0 < piece ? p.n_tok - p.tok0 : piece;
+            if (p.dim <= 64) rc = launch_scan_d<64>(p, n, st);
+            else if (p.dim <= 128) rc = launch_scan_d<128>(p, n, st);
+            else rc = launch_scan_d<256>(p, n, st);
+            if (rc != TBL_OK) return rc;
+        }
+    }
     const cudaError_t e = launch_dependent(delta_out_kernel<T>, dim3(ceil_div(static_cast<long long>(rows) * p.heads, 8)), dim3(256), 0, st, p, rows);
     return e == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
