@@ -74,7 +74,7 @@ struct DeltaParams {
 
 constexpr int kScanLanes = 8;          // groups of sixteen lanes in the consumer warps; each has NC value columns
 constexpr int kScanThreads = 32 * 5;   // four consumer warps, one producer
-constexpr int kStageRounds = 4;        // rounds per bulk copy
+constexpr int kStageRounds = 8;        // rounds per bulk copy
 
 // The scan takes two tokens per round.  With w, u, q = a * u, k, r, v of the two tokens (0 and 1) and the state S before
 // them, everything the round needs from S are four dot products per column, taken together:
@@ -91,7 +91,7 @@ struct Record {
     static constexpr int kValues = kScalars + 16;                      // v of both tokens
     static constexpr int kFloats = kValues + 2 * DKP;
     static constexpr int kStageBytes = 4 * kStageRounds * kFloats;
-    static constexpr int kStages = DKP == 256 ? 4 : 6;                 // bulk copies on their way or in use
+    static constexpr int kStages = DKP == 256 ? 2 : 4;                 // bulk copies on their way or in use
 };
 // Most records of a head at a time: longer sequences are scanned in pieces, more sequences in groups, so that the records
 // between the two kernels stay in L2 (16 heads of 128: 93 MB).
@@ -215,7 +215,10 @@ __global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p,
 }
 
 // What bounds it is a round's chain from the state through the dot products and their sums over sixteen lanes back to the
-// state, so the columns are spread over as many SMs as there are.  Every wait is bounded.
+// state (350 ns a round at 16 columns, of which the vectors' way out of shared memory takes 160), so the columns are spread
+// over as many SMs as there are, and whatever does not wait for the sums is done while they travel.  6001 tokens, 16 heads of
+// 128: 1743 us with the records made by each block of columns for itself on 64 SMs, 1070 now and 75 for the records.
+// Every wait is bounded.
 template <int DKP, int NC>
 __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaParams p, const int stages) {
     using R = Record<DKP>;
@@ -277,22 +280,28 @@ __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaPar
         const bool alive = mbar_wait_bounded(&full[b], (ch / stages) & 1, p.status);
         if (!__all_sync(0xffffffffu, alive)) break;
         const int t0 = 2 * ch * kStageRounds, n_rounds = min(kStageRounds, rounds - ch * kStageRounds);
+        constexpr int V = DKP / 4;                         // 16-byte units per vector
+        ulonglong2 c[4][G];                                // the dot products' vectors, a round ahead
+        auto load_dots = [&](int i) {
+            const ulonglong2* q = reinterpret_cast<const ulonglong2*>(sm + static_cast<size_t>(b * kStageRounds + i) * R::kFloats) + l;
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+#pragma unroll
+                for (int g = 0; g < G; ++g) c[d][g] = q[d * V + 16 * g];
+        };
+        load_dots(0);
 #pragma unroll 1
         for (int i = 0; i < n_rounds; ++i) {
             const float* rec = sm + static_cast<size_t>(b * kStageRounds + i) * R::kFloats;
             const ulonglong2* q = reinterpret_cast<const ulonglong2*>(rec) + l;
-            constexpr int V = DKP / 4;                     // 16-byte units per vector
             float x[4][NC];
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
-                ulonglong2 c[G];
-#pragma unroll
-                for (int g = 0; g < G; ++g) c[g] = q[d * V + 16 * g];
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
-                    pair2 a = mul2(c[0].x, S[n][0].x), e = mul2(c[0].y, S[n][0].y);
+                    pair2 a = mul2(c[d][0].x, S[n][0].x), e = mul2(c[d][0].y, S[n][0].y);
 #pragma unroll
-                    for (int g = 1; g < G; ++g) { a = fma2(c[g].x, S[n][g].x, a); e = fma2(c[g].y, S[n][g].y, e); }
+                    for (int g = 1; g < G; ++g) { a = fma2(c[d][g].x, S[n][g].x, a); e = fma2(c[d][g].y, S[n][g].y, e); }
                     x[d][n] = sum2(add2(a, e));
                 }
             }
@@ -301,6 +310,23 @@ __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaPar
             for (int n = 0; n < NC; ++n) { v0[n] = rec[R::kValues + min(j0 + cl + n, DKP - 1)]; v1[n] = rec[R::kValues + DKP + min(j0 + cl + n, DKP - 1)]; }
             const float4 f = *reinterpret_cast<const float4*>(rec + R::kScalars + 4 * token);
             const float2 fd = *reinterpret_cast<const float2*>(rec + R::kScalars + 8);
+            // what the update does not need the dot products for, while those are on their way through the lanes
+            pair2 p0[NC], p1[NC];
+#pragma unroll
+            for (int n = 0; n < NC; ++n) { p0[n] = dup2(v0[n]); p1[n] = dup2(v1[n]); }
+            ulonglong2 q0[G], q1[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const ulonglong2 w = q[4 * V + 16 * g], k0 = q[5 * V + 16 * g], k1 = q[7 * V + 16 * g];
+                q0[g] = q[6 * V + 16 * g];
+                q1[g] = q[8 * V + 16 * g];
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    S[n][g].x = fma2(k1.x, p1[n], fma2(k0.x, p0[n], mul2(w.x, S[n][g].x)));
+                    S[n][g].y = fma2(k1.y, p1[n], fma2(k0.y, p0[n], mul2(w.y, S[n][g].y)));
+                }
+            }
+            if (i + 1 < n_rounds) load_dots(i + 1);
             float y[2][NC], z[NC], r;
 #pragma unroll
             for (int d = 0; d < 2; ++d)
@@ -326,18 +352,16 @@ __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaPar
             }
 #pragma unroll
             for (int n = 0; n < NC; ++n) d1[n] = fmaf(fd.x, v0[n], fmaf(-fd.y, d0[n], d1[n]));
-            pair2 p0[NC], p1[NC], m0[NC], m1[NC];
+            pair2 m0[NC], m1[NC];
 #pragma unroll
-            for (int n = 0; n < NC; ++n) { p0[n] = dup2(v0[n]); p1[n] = dup2(v1[n]); m0[n] = dup2(-d0[n]); m1[n] = dup2(-d1[n]); }
+            for (int n = 0; n < NC; ++n) { m0[n] = dup2(-d0[n]); m1[n] = dup2(-d1[n]); }
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const ulonglong2 w = q[4 * V + 16 * g], k0 = q[5 * V + 16 * g], q0 = q[6 * V + 16 * g], k1 = q[7 * V + 16 * g], q1 = q[8 * V + 16 * g];
+            for (int g = 0; g < G; ++g)
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
-                    S[n][g].x = fma2(q1.x, m1[n], fma2(k1.x, p1[n], fma2(q0.x, m0[n], fma2(k0.x, p0[n], mul2(w.x, S[n][g].x)))));
-                    S[n][g].y = fma2(q1.y, m1[n], fma2(k1.y, p1[n], fma2(q0.y, m0[n], fma2(k0.y, p0[n], mul2(w.y, S[n][g].y)))));
+                    S[n][g].x = fma2(q1[g].x, m1[n], fma2(q0[g].x, m0[n], S[n][g].x));
+                    S[n][g].y = fma2(q1[g].y, m1[n], fma2(q0[g].y, m0[n], S[n][g].y));
                 }
-            }
             const float out = fmaf(f.x, pick(v0), fmaf(-f.y, pick(d0), fmaf(f.z, pick(v1), fmaf(-f.w, pick(d1), r))));
             if (writes && t0 + 2 * i + token < p.some) o[static_cast<size_t>(t0 + 2 * i) * HD] = out;
         }
@@ -586,9 +610,8 @@ int launch_scan_n(const DeltaParams& p, int n_seq, cudaStream_t st) {
 template <int DKP>
 int launch_scan_d(const DeltaParams& p, int n_seq, cudaStream_t st) {
     auto ctas = [&](int cols) { return static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq; };
-#ifdef SCANNC
-    return launch_scan_n<DKP, SCANNC>(p, n_seq, st);
-#endif
+    // the widest blocks of columns that still take most of the SMs (2000 tokens of 128 channels, 32 / 16 / 8 columns: 32 heads
+    // 547 / 766 / 1159 us; 16 heads 480 / 380 / 580; 8 heads 463 / 364 / 305)
     if (ctas(32) >= 100) return launch_scan_n<DKP, 4>(p, n_seq, st);
     return ctas(16) >= 100 ? launch_scan_n<DKP, 2>(p, n_seq, st) : launch_scan_n<DKP, 1>(p, n_seq, st);
 }

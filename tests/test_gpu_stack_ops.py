@@ -251,6 +251,28 @@ def test_delta_rule_across_scan_and_single_steps(cuda, stack_lib, precision, hea
     assert not states[1].any()                    # nobody touched the third slot
 
 
+@pytest.mark.parametrize("seqs,heads,dim,n", [(1, 1, 12, 2050), (40, 1, 16, 53), (2, 50, 8, 17), (1, 50, 32, 9), (3, 1, 256, 16)])
+def test_delta_scan_in_pieces_and_groups(cuda, stack_lib, seqs, heads, dim, n):
+    """More rounds than the scan takes at a time (one sequence in pieces, many in groups), and each width of a block of columns."""
+    torch, rng = cuda, np.random.default_rng(n)
+    b = Buf(torch)
+    m, w2, w0, norm = delta_mixer(torch, b, heads, dim, 4, rng)
+    hd = heads * dim
+    states = torch.zeros((seqs, heads, dim, dim), device="cuda")
+    proj = (0.8 * rng.standard_normal((seqs * n, 5 * hd + 4))).astype(np.float32)
+    out = torch.full((seqs * n, hd), float("nan"), device="cuda")
+    size = stack_lib.tbl_delta_workspace_bytes(C.byref(m), 0, seqs * n)
+    ws = torch.full((size,), 255, dtype=torch.uint8, device="cuda")
+    assert stack_lib.tbl_delta_forward(C.byref(m), 0, DELTA_SCAN, 1e-3, b.f32(proj), states.data_ptr(), b.i32(range(seqs)), seqs, n,
+                                       out.data_ptr(), ws.data_ptr(), size, stream(torch)) == 0
+    for i in sorted({0, seqs // 2, seqs - 1}):
+        want_states = np.zeros((heads, dim, dim))
+        want = delta_oracle(proj[i * n:(i + 1) * n].astype(np.float64), heads, dim, w2, w0, norm, 1e-3, want_states)
+        assert_close(f64(out)[i * n:(i + 1) * n], want, 2e-5, f"sequence {i}")
+        assert_close(f64(states[i]).transpose(0, 2, 1), want_states, 2e-5, "state")
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 def test_delta_rule_forgets_and_remembers(cuda, stack_lib):
     """Slow decay and no removal keep the first token for 400 tokens; a removal rate of one wipes its direction."""
     torch, rng = cuda, np.random.default_rng(1)
