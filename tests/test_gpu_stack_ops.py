@@ -673,6 +673,19 @@ def test_attention_does_not_depend_on_what_else_is_in_the_batch_or_on_slots(cuda
         assert np.abs(alone - beside).max() <= (0 if route == A_FLASH else 1e-2) * np.abs(alone).max() + 1e-6
 
 
+@pytest.mark.parametrize("seqs", [17, 18, 22])
+def test_attention_stream_by_clusters_of_four(cuda, stack_lib, seqs):
+    """So many sequences that larger clusters would want every place: the same as the SIMT kernel, either side of the limit."""
+    rng = np.random.default_rng(seqs)
+    a, b = (Attention(cuda, stack_lib, ATT["small"], 1, slots=seqs) for _ in range(2))
+    slots = list(range(seqs))
+    history, x = rng.standard_normal((seqs * 390, a.cols)), rng.standard_normal((seqs, a.cols))
+    for m in (a, b):
+        m.forward(A_FLASH, slots, history)
+    got, want = a.forward(A_STREAM, slots, x), b.forward(A_SIMT, slots, x)
+    assert np.abs(got - want).max() <= 1e-2 * np.abs(want).max()            # bf16 outputs, each rounded once
+
+
 def test_attention_reports_a_full_cache(cuda, stack_lib):
     a = Attention(cuda, stack_lib, ATT["small"], 1, capacity=16)
     stack_lib.tbl_device_status(stream(cuda))
