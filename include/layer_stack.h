@@ -154,14 +154,17 @@ size_t tbl_stack_workspace_bytes(const tbl_stack_model* model, int precision, in
  * capacity); a captured step may be replayed while it does.  want_rows_dev int32 [n_want] lists the rows whose
  * logits go to logits_dev fp32 [n_want, vocab] (n_want 0: no logits).  hidden_trace_dev (may be NULL): fp32
  * [n_layers, rows, width], the residual stream after every layer.  state_dev and workspace_dev 256-byte aligned.
- * A sequence past its capacity, or past the rotary table, sets TBL_DEV_CACHE_FULL and its rows are undefined. */
+ * A sequence past its capacity, or past the rotary table, sets TBL_DEV_CACHE_FULL and its rows are undefined.
+ * The model's weights are in place before the call: linear layers request theirs ahead of the kernel before them, so
+ * that work which changes weights has to have finished, not only to be enqueued before on the stream. */
 int tbl_stack_step(const tbl_stack_model* model, int precision, int slots, int capacity, void* state_dev,
                    const int32_t* slots_dev, int n_seq, int n_tok, int context, const int32_t* tokens_dev,
                    const int32_t* want_rows_dev, int n_want, float* logits_dev, float* hidden_trace_dev,
                    void* workspace_dev, size_t workspace_bytes, void* stream);
 
 /* ---- the step's operators, one entry point each ----------------------------------------------------------------
- * Activations `x` have the precision's type (bf16 or fp32), strides in elements. */
+ * Activations `x` have the precision's type (bf16 or fp32), strides in elements.  Everything these read may be the
+ * result of earlier work on the stream, the weights too. */
 
 /* out[m, :] = W x[m, :] + b [+ residual[m, :]], fp32 out (ld = outputs of the view).  route: 0 the kernel the step
  * would take, 1 the SIMT kernel, 2 the GEMV, 3 the tcgen05 GEMM (bf16 only), 4 the row-streaming kernel (bf16 only);

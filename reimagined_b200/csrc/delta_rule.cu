@@ -70,6 +70,7 @@ struct DeltaParams {
     int ld, heads, dim, rank, n_tok;
     int seq0, tok0, some;    // scan kernel: first sequence and token of this launch, and how many tokens of each
     float rate, key_eps, eps;
+    int w_computed;          // host: of w2, as in DenseCall
 };
 
 constexpr int kScanLanes = 8;          // groups of sixteen lanes in the consumer warps; each has NC value columns
@@ -547,7 +548,7 @@ int decay_products(const tbl_delta_mixer& m, const DeltaParams& p, int precision
         return TBL_ERR_CUDA;
     DenseCall c{};
     c.x = th; c.w = static_cast<const bf16*>(m.decay_up.weight); c.ldx = ldt; c.M = rows; c.K = p.rank; c.N = HD;
-    c.out_f32 = z; c.ldo = HD;
+    c.out_f32 = z; c.ldo = HD; c.w_computed = p.w_computed;
     return launch_dense(precision, kDenseAuto, c, st);
 }
 
@@ -657,11 +658,11 @@ int check_delta(const tbl_delta_mixer& m, int width) {
 size_t delta_workspace(const tbl_delta_mixer& m, int precision, int rows) { return carve(m, precision, rows, nullptr).bytes; }
 
 int launch_delta(const tbl_delta_mixer& m, int precision, int route, float eps, const float* proj, float* states,
-                 const int32_t* slots, int n_seq, int n_tok, void* out, void* ws, cudaStream_t st) {
+                 const int32_t* slots, int n_seq, int n_tok, void* out, void* ws, int w_computed, cudaStream_t st) {
     DeltaParams p{};
     p.proj = proj; p.w2 = static_cast<const bf16*>(m.decay_up.weight); p.w0 = m.decay_up.bias; p.norm = m.norm;
     p.states = states; p.slots = slots; p.out = out; p.ld = m.in.outputs; p.heads = m.heads; p.dim = m.dim; p.rank = m.rank;
-    p.n_tok = n_tok; p.rate = m.decay_rate; p.key_eps = m.key_eps; p.eps = eps;
+    p.n_tok = n_tok; p.rate = m.decay_rate; p.key_eps = m.key_eps; p.eps = eps; p.w_computed = w_computed;
     if (route == 0) route = n_tok == 1 ? 2 : 1;
     if (route == 2) {
         if (n_tok != 1) return TBL_ERR_SHAPE;
@@ -693,7 +694,7 @@ int tbl_delta_forward(const tbl_delta_mixer* mixer, int precision, int route, fl
     if (rc != TBL_OK) return rc;
     if (!workspace_dev || workspace_bytes < delta_workspace(*mixer, precision, n_seq * n_tok)) return TBL_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace_dev) & 255) || (reinterpret_cast<uintptr_t>(states_dev) & 15)) return TBL_ERR_ALIGNMENT;
-    return launch_delta(*mixer, precision, route, eps, proj_dev, states_dev, slots_dev, n_seq, n_tok, out_dev, workspace_dev,
+    return launch_delta(*mixer, precision, route, eps, proj_dev, states_dev, slots_dev, n_seq, n_tok, out_dev, workspace_dev, 1,
                         static_cast<cudaStream_t>(stream));
 }
 

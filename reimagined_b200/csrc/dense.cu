@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256) dense_simt_kernel(const DenseCall c) {
 // A warp owns R weight rows (of a gated layer: R / 2 gate rows and their up rows) and walks K in steps of 256 elements,
 // a 16-byte load per lane and row, four to eight such loads a batch and two batches in flight (the kernel is bound by the
 // bytes on their way: with one load a batch 6144 -> 2048 took 18.4 us, now 6.4); the activation rows sit in shared memory as fp32.  The first weight loads are issued
-// before the wait on the preceding kernel of the step.
+// before the wait on the preceding kernel of the step (where that may be writing them the launch is not a dependent one).
 constexpr int kGemvWarps = 8;
 constexpr int kGemvMaxRows = 4;
 constexpr size_t kGemvMaxSmem = 200 * 1024;
@@ -197,8 +197,8 @@ int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
     const size_t smem = sizeof(float) * M * c.K;
     if (allow_smem(dense_gemv_kernel<T, M, R>, smem, done) != cudaSuccess) return TBL_ERR_CUDA;
     const int units = c.pair_cols ? ceil_div(c.pair_cols, R / 2) : ceil_div(c.N, R);
-    return launch_dependent(dense_gemv_kernel<T, M, R>, dim3(ceil_div(units, kGemvWarps)), dim3(32 * kGemvWarps), smem, st, c) ==
-                   cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
+    const dim3 grid(ceil_div(units, kGemvWarps)), block(32 * kGemvWarps);
+    return launch_next(!c.w_computed, dense_gemv_kernel<T, M, R>, grid, block, smem, st, c) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 
 template <typename T, int M>
@@ -288,6 +288,7 @@ int tbl_dense_forward(const tbl_dense_view* view, int precision, int route, cons
     DenseCall c{};
     c.x = x_dev; c.w = static_cast<const bf16*>(view->weight); c.bias = view->bias; c.ldx = ldx;
     c.M = rows; c.K = view->inputs; c.N = view->outputs; c.out_f32 = out_dev; c.ldo = view->outputs; c.residual = residual_dev;
+    c.w_computed = 1;
     return launch_dense(precision, route, c, static_cast<cudaStream_t>(stream));
 }
 
@@ -307,6 +308,7 @@ int tbl_gated_dense_act_forward(const tbl_dense_view* gate_up, int precision, in
     DenseCall c{};
     c.x = x_dev; c.w = static_cast<const bf16*>(gate_up->weight); c.bias = gate_up->bias; c.ldx = ldx;
     c.M = rows; c.K = gate_up->inputs; c.N = gate_up->outputs; c.ldo = ff; c.pair_cols = ff; c.act = activation;
+    c.w_computed = 1;
     if (precision == TBL_BF16) c.out_b16 = static_cast<bf16*>(out_dev); else c.out_f32 = static_cast<float*>(out_dev);
     return launch_dense(precision, route, c, static_cast<cudaStream_t>(stream));
 }

@@ -6,7 +6,8 @@
 // lane % 4) and feeds two MMAs with them.  No shared-memory staging; the activations stay in L1.
 // A CTA's eight warps share WK-way the K range of 8 / WK row units (so that short matrices still fill the GPU); the
 // partial sums meet in shared memory, where the epilogue adds bias and residual, gates, or pairs.  The first weight
-// loads are issued before the wait on the preceding kernel of the step.
+// loads are issued before the wait on the preceding kernel of the step (where that may be writing them the launch is not a
+// dependent one).
 #include "stack.cuh"
 
 namespace tbl {
@@ -124,7 +125,7 @@ cudaError_t launch_u(const DenseCall& c, dim3 grid, int wk, cudaStream_t st) {
     const size_t smem = sizeof(float) * kWarps * TA * 16 * (NB * 8 + 1);
     const cudaError_t e = allow_smem(dense_rows_kernel<TA, NB, U, CTAS>, smem, done);
     if (e != cudaSuccess) return e;
-    return launch_dependent(dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
+    return launch_next(!c.w_computed, dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
 }
 
 template <int TA, int NB>

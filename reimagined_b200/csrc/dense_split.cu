@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
             for (int j = max(0, i - n); j < i; ++j) mbar_wait_bounded(&full[j % n], (j / n) & 1, p.status);
     };
     if (warp == 0) {
-        // the weights depend on no kernel before this one
+        // the weights depend on no kernel before this one, unless the call says so
+        if (lane == 0 && c.w_computed) pdl_wait();
         if (lane == 0) produce(&map_b, smem_b, kB, BN * 128, tn * BN, full_b, empty_b);
         __syncwarp();
     } else if (warp == 2 + kSumWarps + kCutWarps) {

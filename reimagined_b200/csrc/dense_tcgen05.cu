@@ -148,7 +148,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
-    // the weights of the first stages do not depend on the kernel before this one
+    // the weights of the first stages do not depend on the kernel before this one, unless the call says so
     int early = 0;
     if (warp == 0) {
         int row0, tn;

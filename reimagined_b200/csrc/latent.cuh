@@ -21,6 +21,7 @@ struct LatentParams {
     int* status;
     int ld, ldq, cw, H, d, rd, vd, R, q_rank, capacity, rope_positions, n_tok, splits, context;
     float scale, eps;
+    int w_computed;              // host: as in DenseCall, of the mixer's weights
 };
 
 // latent_decode.cu: attention over the latent cache on tensor cores

@@ -300,7 +300,7 @@ int run(const tbl_latent_mixer& m, LatentParams p, const Plan& w, int precision,
     if (launch_dependent(latent_prep_kernel<T>, dim3(rows), dim3(kPrepThreads), 0, st, p) != cudaSuccess) return TBL_ERR_CUDA;
     DenseCall c{};
     c.x = p.cq; c.w = static_cast<const bf16*>(m.uq.weight); c.bias = m.uq.bias; c.ldx = p.ldq; c.M = rows; c.K = p.q_rank;
-    c.N = p.H * (p.d + p.rd); c.ldo = c.N;
+    c.N = p.H * (p.d + p.rd); c.ldo = c.N; c.w_computed = p.w_computed;
     if (w.route == kCacheTensor) c.out_b16 = p.q16; else c.out_f32 = p.q;
     int rc = launch_dense(precision, kDenseAuto, c, st);
     if (rc != TBL_OK) return rc;
@@ -339,7 +339,8 @@ size_t latent_workspace(const tbl_latent_mixer& m, int precision, int n_seq, int
 }
 
 int launch_latent(const tbl_latent_mixer& m, int precision, int route, float eps, const float* proj, void* cache, int capacity,
-                  const int32_t* slots, const int32_t* positions, int n_seq, int n_tok, int context, void* out, void* ws, cudaStream_t st) {
+                  const int32_t* slots, const int32_t* positions, int n_seq, int n_tok, int context, void* out, void* ws, int w_computed,
+                  cudaStream_t st) {
     if (route < kAuto || route > kExpanded) return TBL_ERR_INVALID_ARG;
     if ((route == kCacheTensor && (precision != TBL_BF16 || !latent_tensor_supported(m))) ||
         (route == kExpanded && (precision != TBL_BF16 || !latent_expanded_supported(m))))
@@ -359,7 +360,7 @@ int launch_latent(const tbl_latent_mixer& m, int precision, int route, float eps
     p.ld = m.in.outputs; p.ldq = static_cast<int>(round_up(m.q_rank, 8)); p.cw = latent_cache_width(m);
     p.H = m.heads; p.d = m.dim; p.rd = m.rot_dim; p.vd = m.vdim; p.R = m.kv_rank; p.q_rank = m.q_rank;
     p.capacity = capacity; p.rope_positions = m.rope_positions; p.n_tok = n_tok; p.splits = w.splits; p.context = context;
-    p.scale = m.scale; p.eps = eps;
+    p.scale = m.scale; p.eps = eps; p.w_computed = w_computed;
     return precision == TBL_BF16 ? run<bf16>(m, p, w, precision, n_seq, context, st) : run<float>(m, p, w, precision, n_seq, context, st);
 }
 
@@ -392,7 +393,7 @@ int tbl_latent_forward(const tbl_latent_mixer* mixer, int precision, int route, 
     if (!workspace_dev || workspace_bytes < tbl_latent_workspace_bytes(mixer, precision, n_seq, n_tok, context)) return TBL_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace_dev) & 255) || (reinterpret_cast<uintptr_t>(cache_dev) & 15)) return TBL_ERR_ALIGNMENT;
     return launch_latent(*mixer, precision, route, eps, proj_dev, cache_dev, capacity, slots_dev, positions_dev, n_seq, n_tok, context,
-                         out_dev, workspace_dev, static_cast<cudaStream_t>(stream));
+                         out_dev, workspace_dev, 1, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

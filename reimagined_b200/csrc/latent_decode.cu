@@ -297,6 +297,7 @@ int launch_latent_tensor(const LatentParams& p, int rows, cudaStream_t st) {
     DenseCall a{};              // q' = W_uk^T q, all heads in one launch
     a.x = p.q16; a.w = p.uk_t; a.ldx = p.H * (p.d + p.rd); a.M = rows; a.K = p.d; a.N = p.R;
     a.out_b16 = static_cast<bf16*>(p.qa); a.ldo = p.H * p.R;
+    a.w_computed = p.w_computed;
     a.batch = p.H; a.batch_x = p.d + p.rd; a.batch_w = static_cast<long long>(p.R) * p.d; a.batch_out = p.R;
     int rc = launch_dense(TBL_BF16, kDenseRows, a, st);
     if (rc != TBL_OK) return rc;
@@ -309,6 +310,7 @@ int launch_latent_tensor(const LatentParams& p, int rows, cudaStream_t st) {
     DenseCall v{};              // W_uv and the output gate
     v.x = p.lat; v.w = p.uv; v.ldx = p.H * p.R; v.M = rows; v.K = p.R; v.N = p.vd;
     v.out_b16 = static_cast<bf16*>(p.out); v.ldo = p.H * p.vd;
+    v.w_computed = p.w_computed;
     v.batch = p.H; v.batch_x = p.R; v.batch_w = static_cast<long long>(p.vd) * p.R; v.batch_out = p.vd;
     v.gate = p.proj + p.q_rank + p.R + p.rd; v.ldg = p.ld; v.batch_gate = p.vd;
     return launch_dense(TBL_BF16, kDenseRows, v, st);

@@ -298,6 +298,7 @@ int launch_latent_expanded(const tbl_latent_mixer& m, const LatentParams& p, int
         return TBL_ERR_CUDA;
     DenseCall k{};
     k.x = gathered; k.w = p.uk; k.ldx = p.cw; k.M = n_seq * ctx; k.K = p.R; k.N = p.H * p.d; k.out_b16 = p.keys; k.ldo = k.N;
+    k.w_computed = p.w_computed;
     int rc = launch_dense(TBL_BF16, kDenseTensor, k, st);
     if (rc != TBL_OK) return rc;
     DenseCall v{};

@@ -191,14 +191,14 @@ int tbl_stack_step(const tbl_stack_model* model, int precision, int slots, int c
             int e = linear(l.delta.in, S.h, W, S.proj, nullptr);
             if (e == TBL_OK)
                 e = launch_delta(l.delta, precision, 0, m.norm_eps, S.proj, reinterpret_cast<float*>(state.layer[i]), slots_dev, n_seq, n_tok,
-                                 S.mixed, S.mixer, st);
+                                 S.mixed, S.mixer, 0, st);
             return e == TBL_OK ? linear(l.delta.out, S.mixed, l.delta.heads * l.delta.dim, out, residual) : e;
         }
         if (l.mixer == TBL_MIXER_LATENT_ATTENTION) {
             int e = linear(l.latent.in, S.h, W, S.proj, nullptr);
             if (e == TBL_OK)
                 e = launch_latent(l.latent, precision, 0, m.norm_eps, S.proj, state.layer[i], capacity, slots_dev, state.positions, n_seq, n_tok,
-                                  context, S.mixed, S.mixer, st);
+                                  context, S.mixed, S.mixer, 0, st);
             return e == TBL_OK ? linear(l.latent.out, S.mixed, l.latent.heads * l.latent.vdim, out, residual) : e;
         }
         int e = linear(l.attention.in, S.h, W, S.proj, nullptr);

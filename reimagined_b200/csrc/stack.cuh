@@ -72,18 +72,23 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // Launch as a programmatic dependent of the kernel before it on the stream: the kernel must call pdl_wait() before it
-// touches anything an earlier kernel of the step writes.
+// touches anything an earlier kernel of the step writes.  With `dependent` false an ordinary launch, behind all of them.
 template <typename... Params, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_next(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = dependent ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
     note_launch();
     return e;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    return launch_next(true, kernel, grid, block, smem, st, args...);
 }
 
 // Raises a kernel's dynamic shared memory limit once per device, to what its static shared memory leaves.
@@ -107,7 +112,7 @@ struct DenseCall {
     const bf16* w;           // [N, K], ldw between rows (0: K)
     const float* bias;       // [N] or null
     int ldx, M, K, N, ldw;
-    int w_computed;          // w is what an earlier kernel of the step wrote (tensor-core route only): no load of it before the wait
+    int w_computed;          // an earlier kernel of the stream may still be writing w: no load of it before the wait
     float* out_f32;          // exactly one of the two outputs
     bf16* out_b16;
     int ldo, act;            // act: TBL_ACT_* of a gated pair
@@ -163,14 +168,15 @@ int launch_depth_norm(int precision, const DepthNorm& p, cudaStream_t st);
 
 // ---- delta_rule.cu ----------------------------------------------------------------------------------------------
 size_t delta_workspace(const tbl_delta_mixer& m, int precision, int rows);
+// w_computed: as in DenseCall, of the mixer's own weights
 int launch_delta(const tbl_delta_mixer& m, int precision, int route, float eps, const float* proj, float* states,
-                 const int32_t* slots, int n_seq, int n_tok, void* out, void* ws, cudaStream_t st);
+                 const int32_t* slots, int n_seq, int n_tok, void* out, void* ws, int w_computed, cudaStream_t st);
 
 // ---- latent_attention.cu ------------------------------------------------------------------------------------------
 size_t latent_workspace(const tbl_latent_mixer& m, int precision, int n_seq, int n_tok, int context);
 int launch_latent(const tbl_latent_mixer& m, int precision, int route, float eps, const float* proj, void* cache,
                   int capacity, const int32_t* slots, const int32_t* positions, int n_seq, int n_tok, int context,
-                  void* out, void* ws, cudaStream_t st);
+                  void* out, void* ws, int w_computed, cudaStream_t st);
 int latent_cache_width(const tbl_latent_mixer& m);     // cached numbers per token, padded to 16 bytes of bf16
 // ---- attention.cu --------------------------------------------------------------------------------------------------
 size_t attention_workspace(const tbl_attention_mixer& m, int precision, int n_seq, int n_tok, int context);

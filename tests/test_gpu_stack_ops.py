@@ -176,6 +176,96 @@ def test_dense_fp32_in_three_pieces(cuda, stack_lib, m, k, n, ff, shift):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+class MadeOnTheStream:
+    """A bf16 weight [n, k] that a slow kernel computes, which lets the next ones start beside it and leaves them SMs to do so."""
+
+    def __init__(self, torch, lib, n, k):
+        from reimagined_b200.stack import StackEngine
+        torch.manual_seed(n)
+        self.lib, self.b, self.n, self.k = lib, Buf(torch), n, k
+        gate, up = torch.randn(k, 16384).bfloat16(), torch.randn(k, 16384).bfloat16()
+        self.view, self.x = self.b.view(StackEngine._paired(None, gate, up)), (torch.randn(n, 16384) / 128).bfloat16().cuda()
+        self.weight = torch.zeros((n, k), device="cuda", dtype=torch.bfloat16)
+
+    def same(self, torch, call):
+        """call(): the result, a tensor, of work that reads the weight.  Once behind everything, then right behind the kernel."""
+        results = []
+        for wait in (True, False):
+            self.weight.zero_()
+            torch.cuda.synchronize()
+            assert self.lib.tbl_gated_dense_forward(C.byref(self.view), 1, SIMT, self.x.data_ptr(), 16384, self.n, self.k, self.weight.data_ptr(),
+                                                    stream(torch)) == 0
+            if wait:
+                torch.cuda.synchronize()
+            results.append(call())
+        assert self.weight.abs().sum() > 0 and bool(torch.isfinite(results[0]).all())
+        return torch.equal(*results)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("rows", [1, 4, 16, 64, 300])
+def test_weights_made_by_the_kernel_before(cuda, stack_lib, precision, rows):
+    """A linear layer reads no weight before the work enqueued ahead of it has written it."""
+    from reimagined_b200 import capi
+    torch, made = cuda, MadeOnTheStream(cuda, stack_lib, 256, 512)
+    x = torch.randn(rows, 512, device="cuda").to(torch.bfloat16 if precision else torch.float32)
+    out, gated = torch.zeros(rows, 256, device="cuda"), torch.zeros(rows, 128, device="cuda", dtype=x.dtype)
+    view = capi.DenseView(made.weight.data_ptr(), None, 512, 256)
+
+    def plain():
+        assert stack_lib.tbl_dense_forward(C.byref(view), precision, 0, x.data_ptr(), 512, rows, None, out.data_ptr(), stream(torch)) == 0
+        return out.clone()
+
+    def paired():
+        assert stack_lib.tbl_gated_dense_forward(C.byref(view), precision, 0, x.data_ptr(), 512, rows, 128, gated.data_ptr(), stream(torch)) == 0
+        return gated.clone()
+    assert made.same(torch, plain) and made.same(torch, paired)
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("seqs,n", [(6, 1), (1, 40), (1, 300)])
+def test_mixer_weights_made_by_the_kernel_before(cuda, stack_lib, precision, seqs, n):
+    """The same of the weights inside the mixers: the delta rule's decay projection, latent attention's projections."""
+    torch, rng = cuda, np.random.default_rng(n)
+    dtype = torch.bfloat16 if precision else torch.float32
+    b = Buf(torch)
+    m, *_ = delta_mixer(torch, b, 4, 64, 512, rng)
+    made = MadeOnTheStream(torch, stack_lib, 256, 512)
+    m.decay_up.weight = made.weight.data_ptr()
+    proj, slots = torch.randn(seqs * n, 5 * 256 + 512, device="cuda"), b.i32(range(seqs))
+    size = stack_lib.tbl_delta_workspace_bytes(C.byref(m), precision, seqs * n)
+    ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+
+    out, states = torch.zeros((seqs * n, 256), device="cuda", dtype=dtype), torch.zeros((seqs, 4, 64, 64), device="cuda")
+
+    def delta():
+        assert stack_lib.tbl_delta_forward(C.byref(m), precision, 0, 1e-3, proj.data_ptr(), states.data_ptr(), slots, seqs, n, out.data_ptr(),
+                                           ws.data_ptr(), size, stream(torch)) == 0
+        got = out.clone()
+        states.zero_()
+        return got
+    assert made.same(torch, delta)
+    for name, n_out, k in (("uq", 3 * 64, 64), ("uk", 3 * 48, 80), ("uv", 3 * 80, 80), ("uk_t", 3 * 80, 48)):
+        for route in [CACHE_SIMT] + ([CACHE_TENSOR, EXPANDED] if precision else []):
+            a = Latent(torch, stack_lib, SIZES["small"], precision, slots=6)
+            made = MadeOnTheStream(torch, stack_lib, n_out, k)
+            if name == "uk_t":
+                a.m.uk_t = made.weight.data_ptr()
+            else:
+                getattr(a.m, name).weight = made.weight.data_ptr()
+            pd, sd = torch.randn(seqs * n, a.cols, device="cuda"), b.i32(range(seqs))
+            size = stack_lib.tbl_latent_workspace_bytes(C.byref(a.m), precision, seqs, n, n)
+            scratch, result = torch.zeros(size, dtype=torch.uint8, device="cuda"), torch.zeros((seqs * n, 240), device="cuda", dtype=dtype)
+
+            def latent():
+                assert stack_lib.tbl_latent_forward(C.byref(a.m), precision, route, 1e-4, pd.data_ptr(), a.cache.data_ptr(), a.capacity, sd,
+                                                    a.positions.data_ptr(), seqs, n, n, result.data_ptr(), scratch.data_ptr(), size, stream(torch)) == 0
+                return result.clone()
+            assert made.same(torch, latent), (name, route)
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 # ---- norm and depth average -----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("rows,width,count", [(1, 512, 1), (3, 1000, 12), (40, 90, 5), (2, 4100, 19), (33, 516, 9)])
