@@ -100,12 +100,16 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
 
+    // The limit of a bounded wait is meant for this kernel's own pipeline, so nobody waits for a barrier while the kernel before
+    // still runs: only the weights' producer goes ahead, by the places of its ring.
+    if (warp != 0) pdl_wait();
     // TMA producer: `count` blocks through a ring of n places of `bytes` each
     auto produce = [&](const CUtensorMap* map, uint8_t* ring, int n, int bytes, int row, uint64_t* full, uint64_t* empty) {
         int i = 0;
         bool alive = true;
         for (; i < count; ++i) {
             const int s = i % n;
+            if (i == n) pdl_wait();
             if (i >= n) alive = mbar_wait_bounded(&empty[s], ((i / n) - 1) & 1, p.status);
             if (!alive) break;
             mbar_arrive_expect_tx(&full[s], bytes);
@@ -120,7 +124,6 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
         if (lane == 0) produce(&map_b, smem_b, kB, BN * 128, tn * BN, full_b, empty_b);
         __syncwarp();
     } else if (warp == 2 + kSumWarps + kCutWarps) {
-        pdl_wait();
         if (lane == 0 && p.tma_x) produce(&map_x, smem_x, X, kXBytes, m0, full_x, empty_x);
         __syncwarp();
     } else if (warp == 1) {
@@ -190,7 +193,6 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
         // ---------------- rows of x, cut into three pieces: sixteen lanes a row, four elements each ----------------
         const int w = warp - 2 - kSumWarps, q = lane & 15;
         const float* x = static_cast<const float*>(c.x);
-        if (!p.tma_x) pdl_wait();
         for (int i = 0; i < count; ++i) {
             const int s = i % kA, sx = i % X;
             bool alive = i < kA || mbar_wait_bounded(&empty_a[s], ((i / kA) - 1) & 1, p.status);

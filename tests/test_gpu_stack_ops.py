@@ -176,6 +176,22 @@ def test_dense_fp32_in_three_pieces(cuda, stack_lib, m, k, n, ff, shift):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+def test_dense_fp32_behind_a_long_kernel(cuda, stack_lib):
+    """The time that the kernel before still takes does not count against the limits of this one's waits."""
+    torch = cuda
+    torch.manual_seed(0)
+    b = Buf(torch)
+    k = 1 << 26                                    # one block of the SIMT kernel walks along it for seconds, beside idle SMs
+    long_x, long_out = torch.zeros(k, device="cuda"), torch.zeros(1, device="cuda")
+    long_view = b.view(torch.zeros((1, k), dtype=torch.bfloat16, device="cuda"))
+    x, w, out = torch.randn(64, 512, device="cuda"), torch.randn(96, 512).bfloat16(), torch.full((64, 96), float("nan"), device="cuda")
+    view = b.view(w)
+    assert stack_lib.tbl_dense_forward(C.byref(long_view), 0, SIMT, long_x.data_ptr(), k, 1, None, long_out.data_ptr(), stream(torch)) == 0
+    assert stack_lib.tbl_dense_forward(C.byref(view), 0, 0, x.data_ptr(), 512, 64, None, out.data_ptr(), stream(torch)) == 0
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+    assert_close(f64(out), (x.double() @ w.cuda().double().T).cpu().numpy(), 3e-6)
+
+
 class MadeOnTheStream:
     """A bf16 weight [n, k] that a slow kernel computes, which lets the next ones start beside it and leaves them SMs to do so."""
 
