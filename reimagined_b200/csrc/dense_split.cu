@@ -260,7 +260,7 @@ cudaError_t launch_bn(Params p, cudaStream_t st) {
     // shares of K until the SMs are taken, of at least four blocks each
     p.split = 1;
     while (p.split < kMaxSplit && kblocks >= 8 * p.split &&
-           2LL * p.split * tiles_m * tiles_n <= cluster_room(dense_split_kernel<BN>, 2 * p.split, kThreads, smem_for(BN)))
+           2LL * p.split * tiles_m * tiles_n <= cluster_room<dense_split_kernel<BN>>(2 * p.split, kThreads, smem_for(BN)))
         p.split *= 2;
     return launch_dependent_cluster(dense_split_kernel<BN>, dim3(tiles_n * p.split, tiles_m), p.split, dim3(kThreads), smem_for(BN), st, mx, mb, p);
 }

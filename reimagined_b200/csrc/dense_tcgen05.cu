@@ -364,7 +364,7 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
         if (b > 64 && c.N <= b / 2) continue;
         const long long tiles = tm * ((c.N + b - 1) / b);
         for (int s = 1; s <= kMaxSplit; s *= 2) {
-            if (s > 1 && (kb < 4 * s || tiles * s > cluster_room(dense_tcgen05_kernel<256, false, true>, s, kThreads, smem_for(256)))) break;
+            if (s > 1 && (kb < 4 * s || tiles * s > cluster_room<dense_tcgen05_kernel<256, false, true>>(s, kThreads, smem_for(256)))) break;
             const double blocks = static_cast<double>((tiles + kNumSm - 1) / kNumSm) * ((kb + s - 1) / s);
             const double us = blocks * (0.12 + 0.95e-3 * (a_rows + b)) + (s > 1 ? 1.7 + 3.9e-4 * a_rows * b / s : 0.0);
             if (best == 0.0 || us < best) { best = us; bn = b; split = s; }

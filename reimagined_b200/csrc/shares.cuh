@@ -2,6 +2,8 @@
 // memory, and each finishes a part of the rows -- adds the shares up in their order, then bias, residual or gated pair.
 #pragma once
 
+#include <atomic>
+
 #include "stack.cuh"
 
 namespace tbl {
@@ -82,15 +84,17 @@ __device__ __forceinline__ void finish_shares(const DenseCall& c, uint32_t sums,
 
 // CTAs that run at the same time when they come in clusters of 2, 4 or 8 and take an SM each (a cluster lies within one group
 // of SMs, so that some of these stay empty: 148, 132 and 120 on a B200 with 148 SMs).  One more and the launch takes twice as long.
-template <typename Kernel>
-int cluster_room(Kernel kernel, int cluster, int threads, size_t smem) {
-    static int known[64][4] = {};
+// Asked once for every kernel, device and cluster size; a kernel has one number of threads and bytes.
+template <auto Kernel>
+int cluster_room(int cluster, int threads, size_t smem) {
+    static std::atomic<int> known[64][4];
     int dev = 0;
     cudaGetDevice(&dev);
     const int at = cluster >= 8 ? 3 : (cluster >= 4 ? 2 : (cluster >= 2 ? 1 : 0));
-    if (dev >= 0 && dev < 64 && known[dev][at]) return known[dev][at];
+    if (dev >= 0 && dev < 64)
+        if (const int n = known[dev][at].load(std::memory_order_relaxed)) return n;
     static bool done[64] = {};
-    if (allow_smem(kernel, smem, done) != cudaSuccess) return 0;
+    if (allow_smem(Kernel, smem, done) != cudaSuccess) return 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cluster * kNumSm); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
@@ -98,8 +102,8 @@ int cluster_room(Kernel kernel, int cluster, int threads, size_t smem) {
     attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
-    if (dev >= 0 && dev < 64) known[dev][at] = n * cluster;
+    if (cudaOccupancyMaxActiveClusters(&n, Kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (dev >= 0 && dev < 64) known[dev][at].store(n * cluster, std::memory_order_relaxed);
     return n * cluster;
 }
 
