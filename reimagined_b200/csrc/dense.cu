@@ -225,14 +225,17 @@ bool gemv_supported(const DenseCall& c) {
 }
 
 // Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 16 rows, except that more than eight rows of a
-// long K are better shared out (16 x 12288 x 4096: 32 and 23 us; 8 x 6144 x 2048: 9 and 12), and on small matrices
-// longer (32 x 2048 x 2048: 6.4 and 9.2 us, 32 x 4096 x 4096: 20 and 12, 64 x 1024 x 1024: 6.2 and 6.4, 64 x 2048 x 2048:
-// 10.1 and 8.8).
+// long K are better shared out (16 x 12288 x 4096: 32 and 23 us; 8 x 6144 x 2048: 9 and 12).  Up to 32 rows it does where
+// four or eight warps share K (32 x 512 x 2048: 0.74 of the GEMM's time, 32 x 2048 x 2048 0.80, 32 x 4096 x 2048 0.97; but 1.3
+// .. 2.6 at K of 256 and less, 1.2 at 8192) and the matrix is no more than a wave of blocks (17 x 1024 x 4096 0.96, 17 x 2048 x
+// 4096 1.21, 17 x 512 x 8192 1.15); up to 48 rows with eight warps of the shortest share (48 x 1024 x 2048 0.81, 48 x 768 x
+// 2048 1.31, 48 x 1536 x 1024 1.29).  Beyond that never: 512 x 64 x 2048 takes it 14 us and the GEMM 3.2.
 bool rows_pay(const DenseCall& c) {
     const long long size = static_cast<long long>(c.N) * c.K;
     if (c.batch > 0 || c.M <= 8) return true;
     if (c.M <= 16) return c.K < 2LL * c.N || size < (12 << 20);
-    return c.M <= 32 ? size <= (10 << 20) : c.M * size <= (128 << 20);
+    if (c.M <= 32) return c.K >= 512 && c.K <= 4096 && (c.N <= 2048 || (c.N <= 4096 && c.K <= 1024));
+    return c.M <= 48 && c.K >= 1024 && c.K < 1536 && c.N <= 2048;
 }
 
 }  // namespace
