@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256) dense_simt_kernel(const DenseCall c) {
 // A warp owns R weight rows (of a gated layer: R / 2 gate rows and their up rows) and walks K in steps of 256 elements,
 // a 16-byte load per lane and row, four to eight such loads a batch and two batches in flight (the kernel is bound by the
 // bytes on their way: with one load a batch 6144 -> 2048 took 18.4 us, now 6.4); the activation rows sit in shared memory as fp32.  The first weight loads are issued
-// before the wait on the preceding kernel of the step (where that may be writing them the launch is not a dependent one).
+// before the wait on the preceding kernel of the step, unless that may be writing them.
 constexpr int kGemvWarps = 8;
 constexpr int kGemvMaxRows = 4;
 constexpr size_t kGemvMaxSmem = 200 * 1024;
@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const Dense
             for (int i = 0; i < R; ++i)
                 d[u][i] = k + 256 * u < kv ? __ldcs(reinterpret_cast<const uint4*>(wp[i] + k + 256 * u)) : make_uint4(0, 0, 0, 0);
     };
+    pdl_wait_for_weights(c.w_computed);
     load(w, k_first);
     pdl_launch_dependents();
     pdl_wait();
@@ -198,7 +199,7 @@ int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
     if (allow_smem(dense_gemv_kernel<T, M, R>, smem, done) != cudaSuccess) return TBL_ERR_CUDA;
     const int units = c.pair_cols ? ceil_div(c.pair_cols, R / 2) : ceil_div(c.N, R);
     const dim3 grid(ceil_div(units, kGemvWarps)), block(32 * kGemvWarps);
-    return launch_next(!c.w_computed, dense_gemv_kernel<T, M, R>, grid, block, smem, st, c) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
+    return launch_dependent(dense_gemv_kernel<T, M, R>, grid, block, smem, st, c) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 
 template <typename T, int M>

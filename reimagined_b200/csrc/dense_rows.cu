@@ -6,8 +6,7 @@
 // lane % 4) and feeds two MMAs with them.  No shared-memory staging; the activations stay in L1.
 // A CTA's eight warps share WK-way the K range of 8 / WK row units (so that short matrices still fill the GPU); the
 // partial sums meet in shared memory, where the epilogue adds bias and residual, gates, or pairs.  The first weight
-// loads are issued before the wait on the preceding kernel of the step (where that may be writing them the launch is not a
-// dependent one).
+// loads are issued before the wait on the preceding kernel of the step, unless that may be writing them.
 #include "stack.cuh"
 
 namespace tbl {
@@ -16,9 +15,10 @@ namespace {
 
 constexpr int kWarps = 8;
 
+// (not through the read-only path: those loads may move ahead of the wait for weights that were just written)
 __device__ __forceinline__ uint4 ld_stream(const bf16* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(32 * kWarps, CTAS) dense_rows_kernel(const Den
                 for (int h = 0; h < 2; ++h) d[u][i][h] = ok ? ld_stream(wp[i][h] + (s + u) * 32) : zero;
         }
     };
+    pdl_wait_for_weights(c.w_computed);
     load_w(a, s0);
     pdl_launch_dependents();
     pdl_wait();
@@ -125,7 +126,7 @@ cudaError_t launch_u(const DenseCall& c, dim3 grid, int wk, cudaStream_t st) {
     const size_t smem = sizeof(float) * kWarps * TA * 16 * (NB * 8 + 1);
     const cudaError_t e = allow_smem(dense_rows_kernel<TA, NB, U, CTAS>, smem, done);
     if (e != cudaSuccess) return e;
-    return launch_next(!c.w_computed, dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
+    return launch_dependent(dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
 }
 
 template <int TA, int NB>

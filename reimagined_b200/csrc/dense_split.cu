@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
     };
     if (warp == 0) {
         // the weights depend on no kernel before this one, unless the call says so
-        if (lane == 0 && c.w_computed) pdl_wait();
+        pdl_wait_for_weights(c.w_computed);
         if (lane == 0) produce(&map_b, smem_b, kB, BN * 128, tn * BN, full_b, empty_b);
         __syncwarp();
     } else if (warp == 2 + kSumWarps + kCutWarps) {

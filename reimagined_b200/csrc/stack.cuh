@@ -71,24 +71,25 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Before weights are requested ahead of pdl_wait(): where the kernel before may still be writing them, they wait for it too.
+// (Predicated instructions: a branch costs some kernels registers.)
+__device__ __forceinline__ void pdl_wait_for_weights(int w_computed) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %0, 0;\n@p griddepcontrol.launch_dependents;\n@p griddepcontrol.wait;\n}" ::"r"(w_computed) : "memory");
+}
+
 // Launch as a programmatic dependent of the kernel before it on the stream: the kernel must call pdl_wait() before it
-// touches anything an earlier kernel of the step writes.  With `dependent` false an ordinary launch, behind all of them.
+// touches anything an earlier kernel of the step writes.
 template <typename... Params, typename... Args>
-cudaError_t launch_next(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = dependent ? 1 : 0;
+    cfg.attrs = attr; cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
     note_launch();
     return e;
-}
-
-template <typename... Params, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    return launch_next(true, kernel, grid, block, smem, st, args...);
 }
 
 // Raises a kernel's dynamic shared memory limit once per device, to what its static shared memory leaves.
