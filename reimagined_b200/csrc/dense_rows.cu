@@ -22,11 +22,26 @@ __device__ __forceinline__ uint4 ld_stream(const bf16* p) {
     return v;
 }
 
+// What the kernel reads of a DenseCall.
+struct RowsCall {
+    const void* x;
+    const bf16* w;
+    const float* bias;
+    int ldx, M, K, N, ldw, w_computed;
+    float* out_f32;
+    bf16* out_b16;
+    int ldo, act;
+    const float* residual;
+    int pair_cols, ldg, batch_gate;
+    long long batch_w, batch_x, batch_out;
+    const float* gate;
+};
+
 // TA: 16-row weight tiles per warp (a gated layer: the gate tile and its up tile).  NB: blocks of 8 activation rows.
 // U: steps of 32 per batch of loads, two of which are in flight.  CTAS: CTAs that an SM is to have room for (0: left to
 // the compiler).
 template <int TA, int NB, int U, int CTAS>
-__global__ void __launch_bounds__(32 * kWarps, CTAS) dense_rows_kernel(const DenseCall c, const int wk) {
+__global__ void __launch_bounds__(32 * kWarps, CTAS) dense_rows_kernel(const RowsCall c, const int wk) {
     constexpr int LDP = NB * 8 + 1;
     extern __shared__ float part[];                        // [warps][TA * 16][LDP]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -126,7 +141,9 @@ cudaError_t launch_u(const DenseCall& c, dim3 grid, int wk, cudaStream_t st) {
     const size_t smem = sizeof(float) * kWarps * TA * 16 * (NB * 8 + 1);
     const cudaError_t e = allow_smem(dense_rows_kernel<TA, NB, U, CTAS>, smem, done);
     if (e != cudaSuccess) return e;
-    return launch_dependent(dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, c, wk);
+    const RowsCall r{c.x, c.w, c.bias, c.ldx, c.M, c.K, c.N, c.ldw, c.w_computed, c.out_f32, c.out_b16, c.ldo, c.act, c.residual,
+                     c.pair_cols, c.ldg, c.batch_gate, c.batch_w, c.batch_x, c.batch_out, c.gate};
+    return launch_dependent(dense_rows_kernel<TA, NB, U, CTAS>, grid, dim3(32 * kWarps), smem, st, r, wk);
 }
 
 template <int TA, int NB>

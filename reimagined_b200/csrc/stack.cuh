@@ -134,7 +134,6 @@ bool dense_tensor_supported(const DenseCall& c);
 cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st);
 bool dense_split_supported(const DenseCall& c);
 cudaError_t launch_dense_split(const DenseCall& c, cudaStream_t st);
-static_assert(sizeof(DenseCall) == 128, "with eight bytes more the compiler takes more registers for the row-streaming kernel, and an SM a CTA less");
 
 // ---- stack_glue.cu ----------------------------------------------------------------------------------------------
 struct DepthNorm {
