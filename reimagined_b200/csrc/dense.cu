@@ -77,14 +77,14 @@ __global__ void __launch_bounds__(256) dense_simt_kernel(const DenseCall c) {
 
 // ---- GEMV: 1 .. 4 rows; the weights stream through registers once -------------------------------------------------
 // A warp owns R weight rows (of a gated layer: R / 2 gate rows and their up rows) and walks K in steps of 256 elements,
-// a 16-byte load per lane and row, four to eight such loads a batch and two batches in flight (the kernel is bound by the
-// bytes on their way: with one load a batch 6144 -> 2048 took 18.4 us, now 6.4); the activation rows sit in shared memory as fp32.  The first weight loads are issued
-// before the wait on the preceding kernel of the step, unless that may be writing them.
+// a 16-byte load per lane and row, U steps a batch of loads and two batches in flight; the activation rows sit in shared
+// memory as fp32.  The first weight loads are issued before the wait on the preceding kernel of the step, unless that may be
+// writing them.
 constexpr int kGemvWarps = 8;
 constexpr int kGemvMaxRows = 4;
 constexpr size_t kGemvMaxSmem = 200 * 1024;
 
-template <typename T, int M, int R>
+template <typename T, int M, int R, int U>
 __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const DenseCall c) {
     extern __shared__ __align__(16) float xs[];          // [M][K]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const Dense
     for (int i = 0; i < R; ++i) wp[i] = c.w + static_cast<size_t>(min(rows[i], c.N - 1)) * c.ldw;
     const bool vec = ((c.K | c.ldw) & 7) == 0;
     const int kv = vec ? c.K : 0;
-    constexpr int U = R == 1 ? 8 : (R == 2 ? 2 : 1);      // steps of K per batch of loads
     uint4 w[U][R], wn[U][R];
     const int k_first = lane * 8;
     auto load = [&](uint4 (&d)[U][R], int k) {
@@ -192,14 +191,32 @@ __global__ void __launch_bounds__(32 * kGemvWarps) dense_gemv_kernel(const Dense
     }
 }
 
-template <typename T, int M, int R>
-int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
+template <typename T, int M, int R, int U>
+int launch_gemv_u(const DenseCall& c, cudaStream_t st) {
     static bool done[64] = {};
     const size_t smem = sizeof(float) * M * c.K;
-    if (allow_smem(dense_gemv_kernel<T, M, R>, smem, done) != cudaSuccess) return TBL_ERR_CUDA;
+    if (allow_smem(dense_gemv_kernel<T, M, R, U>, smem, done) != cudaSuccess) return TBL_ERR_CUDA;
     const int units = c.pair_cols ? ceil_div(c.pair_cols, R / 2) : ceil_div(c.N, R);
     const dim3 grid(ceil_div(units, kGemvWarps)), block(32 * kGemvWarps);
-    return launch_dependent(dense_gemv_kernel<T, M, R>, grid, block, smem, st, c) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
+    return launch_dependent(dense_gemv_kernel<T, M, R, U>, grid, block, smem, st, c) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
+}
+
+// One or two rows per warp are bound by the bytes on their way: 6144 -> 2048 at one fp32 row takes 18.4 us with one step a batch
+// and 6.4 with eight.  One step it is where there is no second one and at most a block to an SM (256 -> 256: 1.8 and 1.9 us at
+// two rows), and of two rows per warp where two steps' registers mean another wave of blocks: each wave takes as long as it has
+// blocks to an SM (2048 -> 10304, 644 blocks: three rows 16.2 us in one wave of five and 18.9 in two of three, four rows 24.6 in two
+// of four and 22.3 in two of three).
+template <typename T, int M, int R>
+int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
+    const long long ctas = ceil_div(c.pair_cols ? ceil_div(c.pair_cols, R / 2 > 0 ? R / 2 : 1) : ceil_div(c.N, R), kGemvWarps);
+    if constexpr (R == 1)
+        if (c.K > 256 || ctas > kNumSm) return launch_gemv_u<T, M, 1, 8>(c, st);
+    if constexpr (R == 2) {
+        const int fit = static_cast<int>(227 * 1024 / (sizeof(float) * M * c.K + 1024));     // blocks to an SM by shared memory, and by registers
+        auto cost = [&](int regs) { const long long n = fit < regs ? fit : regs; return n * ((ctas + n * kNumSm - 1) / (n * kNumSm)); };
+        if (c.K >= 512 && cost(M <= 2 ? 4 : 3) <= cost(M <= 2 ? 6 : (M == 3 ? 5 : 4))) return launch_gemv_u<T, M, 2, 2>(c, st);
+    }
+    return launch_gemv_u<T, M, R, 1>(c, st);
 }
 
 template <typename T, int M>
