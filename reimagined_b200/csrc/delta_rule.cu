@@ -94,11 +94,16 @@ struct Record {
     static constexpr int kStageBytes = 4 * kStageRounds * kFloats;
     static constexpr int kStages = DKP == 256 ? 2 : 4;                 // bulk copies on their way or in use
 };
-// Most records of a head at a time: longer sequences are scanned in pieces, more sequences in groups, so that the records
-// between the two kernels stay in L2 (16 heads of 128: 93 MB).
-constexpr int kMaxRounds = 1024;
+// Bytes of records at a time: longer sequences are scanned in pieces, more sequences in groups, so that the records between
+// the two kernels stay in the 126 MB of L2 (16 heads of 128: 1061 rounds of all heads).
+constexpr size_t kRecordBytes = size_t(96) << 20;
 inline int padded_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : 256); }
 inline size_t record_floats(int dim) { return 11 * static_cast<size_t>(padded_dim(dim)) + 16; }
+// rounds of all heads at a time, at least a bulk copy's worth
+inline int max_rounds(int heads, int dim) {
+    const size_t n = kRecordBytes / (sizeof(float) * record_floats(dim) * heads);
+    return n < kStageRounds ? kStageRounds : (n > 1000000 ? 1000000 : static_cast<int>(n));
+}
 
 __device__ __forceinline__ float pick4(const float (&v)[4], int n) {
     const float a = n & 1 ? v[1] : v[0], b = n & 1 ? v[3] : v[2];
@@ -572,7 +577,8 @@ Workspace carve(const tbl_delta_mixer& m, int precision, size_t rows, void* base
     w.o = reinterpret_cast<float*>(take(sizeof(float) * rows * HD));
     w.th = take(e * rows * round_up(m.rank, 8));
     // (up to a round per row: a sequence of an odd number of tokens has half a round more)
-    w.records = reinterpret_cast<float*>(take(sizeof(float) * record_floats(m.dim) * m.heads * (rows < kMaxRounds ? rows : kMaxRounds)));
+    const size_t most = max_rounds(m.heads, m.dim);
+    w.records = reinterpret_cast<float*>(take(sizeof(float) * record_floats(m.dim) * m.heads * (rows < most ? rows : most)));
     return w;
 }
 
@@ -594,14 +600,23 @@ int launch_step(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
     return e == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 
+template <int DKP>
+int scan_stages(int tokens) {
+    const int chunks = ceil_div((tokens + 1) / 2, kStageRounds);
+    return chunks < Record<DKP>::kStages ? chunks : Record<DKP>::kStages;
+}
+// CTAs of the scan that run at once: one or two to an SM, by shared memory
+template <int DKP>
+int scan_room(int tokens) { return 2 * (scan_stages<DKP>(tokens) * Record<DKP>::kStageBytes + 2048) <= 227 * 1024 ? 2 * kNumSm : kNumSm; }
+inline int scan_room(int dim, int tokens) { return dim <= 64 ? scan_room<64>(tokens) : (dim <= 128 ? scan_room<128>(tokens) : scan_room<256>(tokens)); }
+
 template <int DKP, int NC>
 int launch_scan_n(const DeltaParams& p, int n_seq, cudaStream_t st) {
     static bool done[64] = {};
     using R = Record<DKP>;
-    const int chunks = ceil_div((p.some + 1) / 2, kStageRounds), stages = chunks < R::kStages ? chunks : R::kStages;
+    const int stages = scan_stages<DKP>(p.some);
     if (allow_smem(delta_scan_kernel<DKP, NC>, static_cast<size_t>(R::kStages) * R::kStageBytes, done) != cudaSuccess) return TBL_ERR_CUDA;
     const dim3 grid(ceil_div(p.dim, kScanLanes * NC), p.heads, n_seq);
-    if (p.heads > 65535 || n_seq > 65535) return TBL_ERR_SHAPE;
     const long long units = static_cast<long long>(n_seq) * p.heads * ((p.some + 1) / 2);
     if (launch_dependent(delta_records_kernel<DKP>, dim3(ceil_div(units, 8)), dim3(256), 0, st, p, n_seq) != cudaSuccess) return TBL_ERR_CUDA;
     return launch_dependent(delta_scan_kernel<DKP, NC>, grid, dim3(kScanThreads), static_cast<size_t>(stages) * R::kStageBytes, st, p, stages) == cudaSuccess
@@ -610,15 +625,22 @@ int launch_scan_n(const DeltaParams& p, int n_seq, cudaStream_t st) {
 
 template <int DKP>
 int launch_scan_d(const DeltaParams& p, int n_seq, cudaStream_t st) {
-    auto ctas = [&](int cols) { return static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq; };
-    // the widest blocks of columns that still take most of the SMs (2000 tokens of 128 channels, 32 / 16 / 8 columns: 32 heads
-    // 547 / 766 / 1159 us; 16 heads 480 / 380 / 580; 8 heads 463 / 364 / 305)
-    if (ctas(32) >= 100) return launch_scan_n<DKP, 4>(p, n_seq, st);
-    return ctas(16) >= 100 ? launch_scan_n<DKP, 2>(p, n_seq, st) : launch_scan_n<DKP, 1>(p, n_seq, st);
+    // Narrow blocks of columns take less time a round (2000 tokens of 128 channels by 32, 16 and 8 columns: 8 heads 463, 364
+    // and 305 us, in one wave each), a second wave of CTAs as long again (16 heads 480, 380 and 580; 32 heads 547, 766 and
+    // 1159), and two to an SM a fifth longer than one.
+    const int room = scan_room<DKP>(p.some);
+    auto cost = [&](int cols, int us) {
+        const long long ctas = static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq;
+        return (ctas > kNumSm && room > kNumSm ? 6 : 5) * us * ((ctas + room - 1) / room);
+    };
+    const long long wide = cost(32, 480), half = cost(16, 380), narrow = cost(8, 305);
+    if (narrow <= half && narrow <= wide) return launch_scan_n<DKP, 1>(p, n_seq, st);
+    return half <= wide ? launch_scan_n<DKP, 2>(p, n_seq, st) : launch_scan_n<DKP, 4>(p, n_seq, st);
 }
 
 template <typename T>
 int launch_scan(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_seq, void* ws, cudaStream_t st) {
+    if (p.heads > 65535 || n_seq > 65535) return TBL_ERR_SHAPE;
     const int rows = n_seq * p.n_tok;
     const Workspace w = carve(m, precision, rows, ws);
     p.o = w.o;
@@ -628,7 +650,21 @@ int launch_scan(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
     p.records = w.records;
     p.status = device_status_ptr();
     if (!p.status) return TBL_ERR_CUDA;
-    const int piece = p.n_tok < 2 * kMaxRounds ? p.n_tok : 2 * kMaxRounds, group = kMaxRounds / ((piece + 1) / 2);
+    // Whole sequences, as many as there is room for (in whole waves of blocks of 32 columns), or, where that would leave SMs
+    // idle, pieces of enough sequences side by side: a scan takes as long by itself (4 sequences of 1100 tokens, 8 heads of
+    // 128, one after the other: 659 us).
+    const int rounds = (p.n_tok + 1) / 2, most = max_rounds(p.heads, p.dim);
+    const int room = static_cast<int>(scan_room(p.dim, p.n_tok) / (static_cast<long long>(ceil_div(p.dim, 32)) * p.heads)), side = room < 1 ? 1 : room;
+    int group = most / rounds, piece = p.n_tok;
+    if (group >= n_seq) {
+        group = n_seq;
+    } else if (group >= side) {
+        group -= group % side;
+    } else {
+        group = side < n_seq ? side : n_seq;
+        const int per = most / group / kStageRounds * kStageRounds;
+        piece = 2 * (per < kStageRounds ? kStageRounds : per);
+    }
     for (p.seq0 = 0; p.seq0 < n_seq; p.seq0 += group) {
         const int n = n_seq - p.seq0 < group ? n_seq - p.seq0 : group;
         for (p.tok0 = 0; p.tok0 < p.n_tok; p.tok0 += piece) {

@@ -379,6 +379,44 @@ def test_delta_scan_in_pieces_and_groups(cuda, stack_lib, seqs, heads, dim, n):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+@pytest.mark.parametrize("seqs,heads,dim,n,scans", [(10, 2, 128, 1800, 2), (7, 1, 256, 4000, 2), (5, 40, 128, 300, 3), (32, 1, 64, 700, 1), (4, 8, 128, 1100, 1)])
+def test_delta_sequences_side_by_side(cuda, stack_lib, seqs, heads, dim, n, scans):
+    """Sequences of a batch come out as they do alone, bit for bit, whole or in pieces, and are not scanned one after the other."""
+    torch, rng = cuda, np.random.default_rng(n)
+    torch.manual_seed(n)
+    b = Buf(torch)
+    m, *_ = delta_mixer(torch, b, heads, dim, 4, rng)
+    hd = heads * dim
+    proj = 0.8 * torch.randn(seqs, n, 5 * hd + 4, device="cuda")
+    states, out = torch.zeros((seqs, heads, dim, dim), device="cuda"), torch.full((seqs, n, hd), float("nan"), device="cuda")
+    size = stack_lib.tbl_delta_workspace_bytes(C.byref(m), 0, seqs * n)
+    ws = torch.full((size,), 255, dtype=torch.uint8, device="cuda")
+
+    def scan(first, count, states, out):
+        assert stack_lib.tbl_delta_forward(C.byref(m), 0, DELTA_SCAN, 1e-3, proj[first:].data_ptr(), states.data_ptr(), b.i32(range(count)), count, n,
+                                           out.data_ptr(), ws.data_ptr(), size, stream(torch)) == 0
+    before = stack_lib.tbl_launch_count()
+    scan(0, seqs, states, out)
+    assert stack_lib.tbl_launch_count() - before == 3 + 2 * scans             # tanh, decay product, head norm; records and scan each time
+    for i in sorted({0, seqs // 2, seqs - 1}):
+        one, alone = torch.zeros((1, heads, dim, dim), device="cuda"), torch.full((n, hd), float("nan"), device="cuda")
+        scan(i, 1, one, alone)
+        assert torch.equal(one[0], states[i]) and torch.equal(alone, out[i])
+    assert bool(torch.isfinite(out).all()) and stack_lib.tbl_device_status(stream(torch)) == 0
+
+
+def test_delta_scan_refuses_more_sequences_than_a_grid_has(cuda, stack_lib):
+    torch, rng = cuda, np.random.default_rng(0)
+    b = Buf(torch)
+    m, *_ = delta_mixer(torch, b, 1, 4, 1, rng)
+    seqs = 65536
+    proj, states = torch.zeros((seqs, 21), device="cuda"), torch.zeros((seqs, 1, 4, 4), device="cuda")
+    out, size = torch.zeros((seqs, 4), device="cuda"), stack_lib.tbl_delta_workspace_bytes(C.byref(m), 0, seqs)
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    assert stack_lib.tbl_delta_forward(C.byref(m), 0, DELTA_SCAN, 1e-3, proj.data_ptr(), states.data_ptr(), b.i32(range(seqs)), seqs, 1,
+                                       out.data_ptr(), ws.data_ptr(), size, stream(torch)) == -2
+
+
 def test_delta_rule_forgets_and_remembers(cuda, stack_lib):
     """Slow decay and no removal keep the first token for 400 tokens; a removal rate of one wipes its direction."""
     torch, rng = cuda, np.random.default_rng(1)
