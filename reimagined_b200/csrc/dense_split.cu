@@ -1,7 +1,7 @@
 // y[M,N] = x[M,K] (fp32) x w[N,K]^T (bf16) at fp32 accuracy on the 5th-generation tensor cores.
 //
-// An fp32 number is the exact sum of three bf16 numbers (24 bits of significand, cut after 8 and 16), the weights are bf16
-// already and products of two bf16 are exact in fp32: three MMAs per step of K give every product exactly.  What remains is
+// An fp32 number down to 2^-110 is the exact sum of three bf16 numbers (24 bits of significand, cut after 8 and 16), the weights
+// are bf16 already and products of two bf16 are exact in fp32: three MMAs per step of K give every product exactly.  What remains is
 // the accumulation, and there the tensor cores cut off what an addend or the sum loses in alignment, always towards zero.
 // So no accumulator runs for long: the high parts have one of their own, both are taken over into registers after every
 // kSlab blocks of K, where the sums are ordinary rounded fp32 additions.
@@ -11,9 +11,10 @@
 // rows of x up and store the three pieces as 128-byte-swizzled operand rows.  (x comes by TMA too: the fence behind the
 // stores waits for all loads its warp has under way, so that loads ahead of their time would be waited for at once.)  At the end the sums of all shares meet in shared
 // memory (distributed, in the order of the shares) and all warps finish the rows: bias, residual, gated pair.
-// A sum that is not finite is worked out once more the plain way, since infinities have no such pieces.
-// 251 x 6144 x 2048: 58 us (0.33 PFLOP/s of bf16 MMAs), the SIMT kernel 700 us; relative error 1.5e-7, the SIMT kernel's
-// 1.4e-6.  What bounds it is the round of a block through the cutting warps, their fence and the MMAs with two places for
+// A sum that is not finite is worked out once more the plain way, since infinities have no such pieces, and so is a small one of
+// rows some number of which lost bits below bf16's smallest.
+// 251 x 6144 x 2048: 58 us (0.33 PFLOP/s of bf16 MMAs), one of them for watching the lost bits; the SIMT kernel 700 us; relative
+// error 1.5e-7, the SIMT kernel's 1.4e-6.  What bounds it is the round of a block through the cutting warps, their fence and the MMAs with two places for
 // the pieces: 1.2 us a block of 64, where the MMAs alone take 0.3.
 // Every wait is bounded: on a timeout the role records the status word and falls through to the common exit.
 #include <cuda.h>
@@ -53,14 +54,22 @@ struct Params {
 __device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 __device__ __forceinline__ float beyond_bf16(float v) { return v - __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
 
-__device__ __noinline__ float plain_product(const DenseCall& c, int m, int n) {
+// Bits that the pieces of a row lost are worth less than K * 2^-133 * |w|: nothing beside a sum from here on, for weights up to 2^50.
+constexpr float kSmallSum = 9.094947e-13f;                 // 2^-40
+
+// lost: address of the flag of these rows, one per share of K
+__device__ __noinline__ float rechecked(const DenseCall& c, int m, int n, float sum, uint32_t lost, int split) {
+    if (fabsf(sum) < kSmallSum) {
+        uint32_t any = 0;
+        for (int k = 0; k < split; ++k) any |= peer_load_u32(lost, k);
+        if (!any) return sum;
+    }
     const float* x = static_cast<const float*>(c.x) + static_cast<size_t>(m) * c.ldx;
     const bf16* w = c.w + static_cast<size_t>(n) * c.ldw;
     float v = 0.0f;
     for (int k = 0; k < c.K; ++k) v = fmaf(x[k], to_f(w[k]), v);
     return v;
 }
-__device__ __forceinline__ float checked(const DenseCall& c, int m, int n, float v) { return fabsf(v) <= 3.402823466e38f || n >= c.N ? v : plain_product(c, m, n); }
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Params p) {
@@ -75,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
     uint64_t* full_a = reinterpret_cast<uint64_t*>(smem_x + X * kXBytes);
     uint64_t *empty_a = full_a + kA, *full_b = empty_a + kA, *empty_b = full_b + kB, *full_x = empty_b + kB, *empty_x = full_x + X,
              *tmem_full = empty_x + X, *tmem_empty = tmem_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2), *lost_rows = tmem_slot + 1;     // [cutting warps]
     const DenseCall& c = p.c;
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int share = blockIdx.x % p.split, tn = blockIdx.x / p.split, m0 = blockIdx.y * BM;
@@ -193,14 +202,16 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
         // ---------------- rows of x, cut into three pieces: sixteen lanes a row, four elements each ----------------
         const int w = warp - 2 - kSumWarps, q = lane & 15;
         const float* x = static_cast<const float*>(c.x);
+        uint32_t lost = 0;                                             // low halves of third pieces: bits that those do not hold
         for (int i = 0; i < count; ++i) {
             const int s = i % kA, sx = i % X;
             bool alive = i < kA || mbar_wait_bounded(&empty_a[s], ((i / kA) - 1) & 1, p.status);
             if (alive && p.tma_x) alive = mbar_wait_bounded(&full_x[sx], (i / X) & 1, p.status);
             if (!__all_sync(0xffffffffu, alive)) break;
-            if (m0 + w * 16 < c.M || i < kA) {                         // (rows past the end stay zero)
+            float4 v[8];
+            const bool live = m0 + w * 16 < c.M || i < kA;             // (rows past the end stay zero)
+            if (live) {
                 uint8_t* dst = smem + s * 3 * kPieceBytes;
-                float4 v[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int r = w * 16 + 2 * j + (lane >> 4), k = (kb0 + i) * BKE + 4 * q;
@@ -221,7 +232,10 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
                         const int r = w * 16 + 2 * j + (lane >> 4);
                         *reinterpret_cast<uint2*>(dst + piece * kPieceBytes + r * 128 + (((q >> 1) ^ (r & 7)) << 4) + (q & 1) * 8) =
                             make_uint2(high_halves(v[j].x, v[j].y), high_halves(v[j].z, v[j].w));
-                        v[j] = make_float4(beyond_bf16(v[j].x), beyond_bf16(v[j].y), beyond_bf16(v[j].z), beyond_bf16(v[j].w));
+                        if (piece == 2)
+                            lost |= __float_as_uint(v[j].x) | __float_as_uint(v[j].y) | __float_as_uint(v[j].z) | __float_as_uint(v[j].w);
+                        else
+                            v[j] = make_float4(beyond_bf16(v[j].x), beyond_bf16(v[j].y), beyond_bf16(v[j].z), beyond_bf16(v[j].w));
                     }
             }
             fence_proxy_async();
@@ -231,12 +245,18 @@ __global__ void __launch_bounds__(kThreads, 1) dense_split_kernel(const __grid_c
                 if (p.tma_x) mbar_arrive(&empty_x[sx]);
             }
         }
+        lost = __any_sync(0xffffffffu, (lost & 0xffff) != 0);
+        if (lane == 0) lost_rows[w] = lost;
     }
 
     // ---------------- all shares' sums, a part of the rows per CTA ----------------
     pdl_wait();
     if (p.split > 1) cluster_sync_all(); else __syncthreads();
-    finish_shares<BN, LDS, kThreads>(c, smem_u32(smem), p.split, share, tn, m0, BM, p.vec_out, [&](int m, int n, float v) { return checked(c, m, n, v); });
+    const uint32_t lost_at = smem_u32(lost_rows);
+    finish_shares<BN, LDS, kThreads>(c, smem_u32(smem), p.split, share, tn, m0, BM, p.vec_out, [&](int m, int n, float v) {
+        const float size = fabsf(v);
+        return (size >= kSmallSum && size <= 3.402823466e38f) || n >= c.N ? v : rechecked(c, m, n, v, lost_at + 4 * ((m - m0) >> 4), p.split);
+    });
     // nobody leaves while a neighbour may still read its sums; then the allocating warp releases TMEM
     tc_fence_before();
     if (p.split > 1) cluster_sync_all(); else __syncthreads();

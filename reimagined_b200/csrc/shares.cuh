@@ -19,6 +19,12 @@ __device__ __forceinline__ float4 peer_load(uint32_t addr, int rank) {
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t peer_load_u32(uint32_t addr, int rank) {
+    uint32_t a, v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
 
 // `sums`: shared-memory address of this tile's sums, LDS floats per row, the same in every CTA of the cluster.  vec: outputs
 // and residual take accesses of four columns.  check(m, weight row, sum) returns the sum to use.

@@ -176,6 +176,31 @@ def test_dense_fp32_in_three_pieces(cuda, stack_lib, m, k, n, ff, shift):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+@pytest.mark.parametrize("m,k,n,shift", [(16, 256, 64, 0), (130, 4096, 40, 0), (5, 72, 9, 1), (9, 2112, 63, 0)])
+def test_dense_fp32_of_numbers_too_small_for_pieces(cuda, stack_lib, m, k, n, shift):
+    """Below 2^-110 the third piece falls under bf16's smallest number: nothing is lost against the SIMT kernel, also where only some
+    rows, or some numbers of a row, are so small, and rows of zeros stay zeros."""
+    torch = cuda
+    torch.manual_seed(m)
+    b = Buf(torch)
+    w = torch.randn(n, k).bfloat16()
+    view, call = b.view(w), lambda route, x, out: stack_lib.tbl_dense_forward(C.byref(view), 0, route, x.data_ptr(), k + shift, m, None, out.data_ptr(), stream(torch))
+    for down in (108, 114, 121, 127, 133, 140, 147):
+        x = torch.randn(m, k + shift, dtype=torch.float64, device="cuda")
+        x[: m // 2] *= 2.0 ** -down
+        x[m // 2, ::3] *= 2.0 ** -down
+        x[m - 1] = 0
+        x = x.float()
+        out, plain = (torch.full((m, n), float("nan"), device="cuda") for _ in range(2))
+        assert call(0, x, out) == 0 and call(SIMT, x, plain) == 0
+        want, size = (x[:, :k].double() @ w.cuda().double().T, x[:, :k].abs().double() @ w.cuda().abs().double().T)
+        # as for ordinary numbers, and half of the smallest fp32 number for each of the SIMT kernel's additions
+        assert bool(((out.double() - want).abs() <= 2.0 ** -18 * size + k * 2.0 ** -150).all())
+        norm = lambda t: float((t.double() - want)[: m // 2].norm())
+        assert norm(out) <= 1.01 * norm(plain) and not out[m - 1].any()
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 def test_dense_fp32_behind_a_long_kernel(cuda, stack_lib):
     """The time that the kernel before still takes does not count against the limits of this one's waits."""
     torch = cuda
