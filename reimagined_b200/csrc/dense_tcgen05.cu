@@ -206,26 +206,21 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         umma_f16(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), idesc, (kb | kk) != 0 ? 1u : 0u);
                     umma_commit(&empty[s]);
                 }
-                if (alive && kblocks > 0) umma_commit(&tmem_full[buf]);
+                if (alive) umma_commit(&tmem_full[buf]);
             }
         }
     } else if (SHARED) {
         // ---------------- sums of this share into the place of the stages (all of which the MMAs have read) ----------------
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * LDS + half * (BN / 2);
-        bool alive = kblocks == 0 || mbar_wait_bounded(&tmem_full[0], 0, p.status);
+        bool alive = mbar_wait_bounded(&tmem_full[0], 0, p.status);     // (no share is empty: K has four blocks for each)
         alive = __all_sync(0xffffffffu, alive);
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < BN / 2; j += 32) {
             uint32_t r[32];
-            if (kblocks > 0) {
-                tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2) + j, r);
-                tmem_ld_wait();
-            } else {
-#pragma unroll
-                for (int e = 0; e < 32; ++e) r[e] = 0;
-            }
+            tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2) + j, r);
+            tmem_ld_wait();
             if (alive)
 #pragma unroll
                 for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(row + j + e) = make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);

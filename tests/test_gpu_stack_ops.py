@@ -90,9 +90,12 @@ def test_dense_tall_tiles_and_the_residual_in_place(cuda, stack_lib):
 
 
 @pytest.mark.parametrize("m,k,n,ff", [(1, 512, 8, 8), (64, 1024, 130, 70), (65, 520, 2050, 1000), (128, 4104, 257, 97), (129, 8192, 64, 32),
-                                      (512, 3072, 1024, 1030), (700, 1032, 1026, 515)])
+                                      (512, 3072, 1024, 1030), (700, 1032, 1026, 515),
+                                      (1, 1544, 8, 8), (65, 2056, 2050, 1000), (500, 6152, 2050, 1030), (512, 6144, 2048, 1024), (700, 4104, 1026, 515)])
 def test_dense_shares_of_k(cuda, stack_lib, m, k, n, ff):
-    """Few tiles and a long K: the CTAs of a cluster share a tile's K (two or four shares, the last one short) and its rows."""
+    """Few tiles and a long K: the CTAs of a cluster share a tile's K (two or four shares, the last one short) and its rows.  By the
+    cost that launch_dense_tensor() works out, tiles are 64 columns wide, for 512 and 500 rows 128, for the last two 256; the first,
+    the third and (700, 1032) are not shared and stand beside the others."""
     from reimagined_b200.stack import StackEngine
     torch, rng = cuda, np.random.default_rng(m * k + n)
     b = Buf(torch)
@@ -111,9 +114,11 @@ def test_dense_shares_of_k(cuda, stack_lib, m, k, n, ff):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
-@pytest.mark.parametrize("m,k,n", [(1, 264, 148 * 16), (1, 5000, 148 * 16 + 1), (8, 512, 1200), (16, 520, 148 * 64), (9, 520, 148 * 64 + 9), (3, 264, 32000), (16, 2056, 37888)])
+@pytest.mark.parametrize("m,k,n", [(1, 264, 148 * 16), (1, 5000, 148 * 16 + 1), (8, 512, 1200), (16, 520, 148 * 64), (9, 520, 148 * 64 + 9), (3, 264, 32000), (16, 2056, 37888),
+                                   (1, 5000, 148 * 16 - 7), (8, 4104, 148 * 16 - 7), (9, 2056, 37889), (16, 2056, 37889)])
 def test_dense_rows_by_the_number_of_blocks(cuda, stack_lib, m, k, n):
-    """Row-streaming kernel: one block to an SM and a long K, two, three, four blocks to an SM, and one more than a wave."""
+    """Row-streaming kernel: one block to an SM and a long K (148 blocks at N 2361), two, three, four blocks to an SM, and one more
+    than a wave (297 blocks of two weight tiles per warp at N 37889)."""
     torch = cuda
     torch.manual_seed(n)
     b = Buf(torch)
@@ -122,6 +127,34 @@ def test_dense_rows_by_the_number_of_blocks(cuda, stack_lib, m, k, n):
     assert stack_lib.tbl_dense_forward(C.byref(b.view(w)), 1, ROWS, x.data_ptr(), k, m, None, out.data_ptr(), stream(torch)) == 0
     want = x.double() @ w.cuda().double().T
     assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("m,k,ff", [(9, 520, 9593), (16, 1032, 9593), (16, 264, 18945)])
+def test_gated_dense_rows_beyond_two_blocks_to_an_sm(cuda, stack_lib, m, k, ff):
+    """300, 600 and 297 blocks of the row-streaming kernel, ragged at the end of K and of the outputs."""
+    from reimagined_b200.stack import StackEngine
+    torch = cuda
+    torch.manual_seed(ff)
+    b = Buf(torch)
+    x, gate, up = torch.randn(m, k).bfloat16().cuda(), *(((torch.randn(ff, k) * k ** -0.5).bfloat16()) for _ in range(2))
+    out = torch.full((m, ff), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert stack_lib.tbl_gated_dense_forward(C.byref(b.view(StackEngine._paired(None, gate, up))), 1, ROWS, x.data_ptr(), k, m, ff, out.data_ptr(),
+                                             stream(torch)) == 0
+    gw, uw = (x.double() @ t.cuda().double().T for t in (gate, up))
+    assert_close(f64(out), (torch.nn.functional.silu(gw) * uw).cpu().numpy(), 4e-3)
+
+
+@pytest.mark.parametrize("m,k,n", [(33, 512, 2048), (49, 1024, 1024), (65, 1024, 512), (128, 512, 640), (512, 576, 256), (900, 512, 130)])
+def test_dense_of_many_rows_is_the_gemm(cuda, stack_lib, m, k, n):
+    """However small the matrix: the row-streaming kernel takes several times as long there."""
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, view, outs = torch.randn(m, k).bfloat16().cuda(), b.view(torch.randn(n, k).bfloat16()), []
+    for route in (0, TENSOR, ROWS):
+        outs.append(torch.full((m, n), float("nan"), device="cuda"))
+        assert stack_lib.tbl_dense_forward(C.byref(view), 1, route, x.data_ptr(), k, m, None, outs[-1].data_ptr(), stream(torch)) == 0
+    assert torch.equal(outs[0], outs[1]) and not torch.equal(outs[0], outs[2])           # (the two add up in different orders)
 
 
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
@@ -142,9 +175,10 @@ def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
     assert_close(f64(out), want, 4e-3 if precision else 3e-6)
 
 
-@pytest.mark.parametrize("m,k,n,ff,shift", [(5, 8, 1, 1, 0), (127, 72, 65, 33, 0), (129, 512, 64, 96, 1), (16, 1032, 130, 250, 0), (257, 4096, 63, 31, 0), (6, 1088, 12900, 6500, 0)])
+@pytest.mark.parametrize("m,k,n,ff,shift", [(5, 8, 1, 1, 0), (127, 72, 65, 33, 0), (129, 512, 64, 96, 1), (16, 1032, 130, 250, 0), (257, 4096, 63, 31, 0), (6, 1088, 12900, 6500, 0),
+                                           (16, 2112, 63, 31, 0)])
 def test_dense_fp32_in_three_pieces(cuda, stack_lib, m, k, n, ff, shift):
-    """fp32 rows on the tensor cores: one to eight shares of K, rows of x that start on 16 bytes and that do not, gated pairs, and
+    """fp32 rows on the tensor cores: one to eight shares of K (the last of them empty at K 2112), rows of x that start on 16 bytes and that do not, gated pairs, and
     rows with infinities, NaN and numbers near the end of the range, which have no three pieces."""
     from reimagined_b200.stack import StackEngine
     torch, rng = cuda, np.random.default_rng(m + n)
