@@ -8,7 +8,7 @@
 //   delta_records_kernel  turns the raw projections of two tokens into a record: everything a round of the scan multiplies
 //                       with, once per head instead of once per block of columns.
 //   delta_scan_kernel   a sequence of tokens, two per round: a CTA owns 8, 16 or 32 columns of a head.  A producer brings the
-//                       records by bulk copies, four warps walk them with the state in registers.
+//                       records by bulk copies (or, of short sequences, eight make them), four warps walk them with the state in registers.
 //   delta_step_kernel   one token: a CTA per head also computes the low-rank decay product, the head norm and the gate.
 #include "stack.cuh"
 
@@ -74,8 +74,11 @@ struct DeltaParams {
 };
 
 constexpr int kScanLanes = 8;          // groups of sixteen lanes in the consumer warps; each has NC value columns
-constexpr int kScanThreads = 32 * 5;   // four consumer warps, one producer
+// warps beside the four consumers: one that starts bulk copies, or as many to make records as there are registers for
+__host__ __device__ constexpr int producers(int dkp, int nc, bool own) { return !own ? 1 : (dkp == 256 && nc == 4 ? 4 : 8); }
+__host__ __device__ constexpr int scan_threads(int dkp, int nc, bool own) { return 32 * (4 + producers(dkp, nc, own)); }
 constexpr int kStageRounds = 8;        // rounds per bulk copy
+constexpr int kOwnTokens = 32;         // most tokens of a sequence whose records the scan makes itself
 
 // The scan takes two tokens per round.  With w, u, q = a * u, k, r, v of the two tokens (0 and 1) and the state S before
 // them, everything the round needs from S are four dot products per column, taken together:
@@ -94,8 +97,9 @@ struct Record {
     static constexpr int kStageBytes = 4 * kStageRounds * kFloats;
     static constexpr int kStages = DKP == 256 ? 2 : 4;                 // bulk copies on their way or in use
 };
-// Bytes of records at a time: longer sequences are scanned in pieces, more sequences in groups, so that the records between
-// the two kernels stay in the 126 MB of L2 (16 heads of 128: 1061 rounds of all heads).
+// Bytes of records at a time: longer sequences are scanned in pieces, more sequences in groups, so that the workspace stays small and
+// the records mostly in the 126 MB of L2 (16 heads of 128: 1104 rounds of all heads; by twice the bytes 6001 tokens of 32 heads take
+// 1577 us, by these 1584).
 constexpr size_t kRecordBytes = size_t(96) << 20;
 inline int padded_dim(int dim) { return dim <= 64 ? 64 : (dim <= 128 ? 128 : 256); }
 inline size_t record_floats(int dim) { return 11 * static_cast<size_t>(padded_dim(dim)) + 16; }
@@ -114,19 +118,13 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf
 // (a division good to two units in the last place)
 __device__ __forceinline__ float sigmoid_near(float z) { return __fdividef(1.0f, 1.0f + expf(-z)); }
 
-// One warp per record; lane l has channels 4l .. 4l + 3 (+ 128).
+// The record of a head's tokens at row `at` and, where `second`, the one behind it, by one warp; lane l has channels 4l .. 4l + 3
+// (+ 128).
 template <int DKP>
-__global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p, const int n_seq) {
+__device__ __forceinline__ void make_record(const DeltaParams& p, int head, size_t at, bool second, float* rec) {
     using R = Record<DKP>;
     constexpr int NI = (DKP + 127) / 128;      // groups of four channels per lane
-    const int lane = threadIdx.x & 31, dim = p.dim, HD = p.heads * dim, rounds = (p.some + 1) / 2;
-    // neighbouring warps take neighbouring heads of the same tokens: their rows are one piece of memory
-    const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const int head = static_cast<int>(unit % p.heads);
-    const size_t at = unit / p.heads;
-    const int seq = static_cast<int>(at / rounds), t0 = 2 * static_cast<int>(at - static_cast<size_t>(seq) * rounds);
-    pdl_launch_dependents();
-    if (seq >= n_seq) return;
+    const int lane = threadIdx.x & 31, dim = p.dim, HD = p.heads * dim;
     const bool vec = ((dim | p.ld) & 3) == 0;          // every row and head starts on 16 bytes
     auto load4 = [&](const float* base, int c, bool live) {
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -138,16 +136,13 @@ __global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p,
         if (c + 3 < dim) v.w = base[c + 3];
         return v;
     };
-    pdl_wait();
-    const bool second = t0 + 1 < p.some;
     float4 r[2][NI], k[2][NI], u[2][NI], q[2][NI], w[2][NI], v[2][NI];
     float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const bool live = s == 0 || second;
-        const size_t row_at = static_cast<size_t>(p.seq0 + seq) * p.n_tok + p.tok0 + t0 + (live ? s : 0);
-        const float* row = p.proj + row_at * p.ld + head * dim;
-        const float* zr = p.z + row_at * HD + head * dim;
+        const float* row = p.proj + (at + (live ? s : 0)) * p.ld + head * dim;
+        const float* zr = p.z + (at + (live ? s : 0)) * HD + head * dim;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
             const int c = 4 * lane + 128 * i;
@@ -176,7 +171,6 @@ __global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p,
             w[s][i] = make_float4(decay(z.x + w0.x), decay(z.y + w0.y), decay(z.z + w0.z), decay(z.w + w0.w));
             if (s == 1 && !second) w[s][i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         }
-    float* rec = p.records + ((static_cast<size_t>(seq) * p.heads + head) * rounds + t0 / 2) * R::kFloats;
     float m[8] = {};
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
@@ -220,13 +214,29 @@ __global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p,
     if (lane < 6) sc[10 + lane] = 0.0f;
 }
 
+template <int DKP>
+__global__ void __launch_bounds__(256) delta_records_kernel(const DeltaParams p, const int n_seq) {
+    const int rounds = (p.some + 1) / 2;
+    // neighbouring warps take neighbouring heads of the same tokens: their rows are one piece of memory
+    const size_t unit = static_cast<size_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    const int head = static_cast<int>(unit % p.heads);
+    const size_t round = unit / p.heads;
+    const int seq = static_cast<int>(round / rounds), t0 = 2 * static_cast<int>(round - static_cast<size_t>(seq) * rounds);
+    pdl_launch_dependents();
+    if (seq >= n_seq) return;
+    pdl_wait();
+    make_record<DKP>(p, head, static_cast<size_t>(p.seq0 + seq) * p.n_tok + p.tok0 + t0, t0 + 1 < p.some,
+                     p.records + ((static_cast<size_t>(seq) * p.heads + head) * rounds + t0 / 2) * Record<DKP>::kFloats);
+}
+
 // What bounds it is a round's chain from the state through the dot products and their sums over sixteen lanes back to the
 // state (350 ns a round at 16 columns, of which the vectors' way out of shared memory takes 160), so the columns are spread
 // over as many SMs as there are, and whatever does not wait for the sums is done while they travel.  6001 tokens, 16 heads of
 // 128: 1743 us with the records made by each block of columns for itself on 64 SMs, 1070 now and 75 for the records.
 // Every wait is bounded.
-template <int DKP, int NC>
-__global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaParams p, const int stages) {
+// OWN: the records are not in memory, warps of the CTA make them where the bulk copies would leave them.
+template <int DKP, int NC, bool OWN>
+__global__ void __launch_bounds__(scan_threads(DKP, NC, OWN)) delta_scan_kernel(const DeltaParams p, const int stages) {
     using R = Record<DKP>;
     constexpr int COLS = kScanLanes * NC;      // value columns per CTA
     constexpr int G = DKP / 64;                // groups of four keys per consumer lane: 4 (l + 16 g), l = lane % 16
@@ -238,13 +248,27 @@ __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(const DeltaPar
     const int rounds = (p.some + 1) / 2, chunks = (rounds + kStageRounds - 1) / kStageRounds;
     const size_t row0 = static_cast<size_t>(p.seq0 + seq) * p.n_tok + p.tok0;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        for (int s = 0; s < stages; ++s) { mbar_init(&full[s], producers(DKP, NC, OWN)); mbar_init(&empty[s], 4); }
         fence_mbar_init();
         fence_proxy_async();
     }
     __syncthreads();
     pdl_launch_dependents();
     pdl_wait();
+    if (OWN && warp >= 4) {
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int s = ch % stages, n = min(kStageRounds, rounds - ch * kStageRounds);
+            const bool alive = ch < stages || mbar_wait_bounded(&empty[s], ((ch / stages) - 1) & 1, p.status);
+            if (!__all_sync(0xffffffffu, alive)) break;
+            for (int i = warp - 4; i < n; i += producers(DKP, NC, OWN)) {
+                const int t0 = 2 * (ch * kStageRounds + i);
+                make_record<DKP>(p, head, row0 + t0, t0 + 1 < p.some, sm + static_cast<size_t>(s * kStageRounds + i) * R::kFloats);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+        return;
+    }
     if (warp == 4) {
         if (lane == 0) {
             const float* src = p.records + (static_cast<size_t>(seq) * p.heads + head) * rounds * R::kFloats;
@@ -605,22 +629,23 @@ int scan_stages(int tokens) {
     const int chunks = ceil_div((tokens + 1) / 2, kStageRounds);
     return chunks < Record<DKP>::kStages ? chunks : Record<DKP>::kStages;
 }
-// CTAs of the scan that run at once: one or two to an SM, by shared memory
-template <int DKP>
-int scan_room(int tokens) { return 2 * (scan_stages<DKP>(tokens) * Record<DKP>::kStageBytes + 2048) <= 227 * 1024 ? 2 * kNumSm : kNumSm; }
-inline int scan_room(int dim, int tokens) { return dim <= 64 ? scan_room<64>(tokens) : (dim <= 128 ? scan_room<128>(tokens) : scan_room<256>(tokens)); }
+// CTAs of the scan that run at once: one or two to an SM, by shared memory.  (Short sequences leave room for more, but gain
+// nothing by it: 16 heads of 128, 24 tokens, 17.5 us by 128 CTAs of 16 columns and 22.5 by 256 of eight.)
+constexpr int scan_room(int dkp) { return dkp <= 64 ? 2 * kNumSm : kNumSm; }
 
-template <int DKP, int NC>
+template <int DKP, int NC, bool OWN>
 int launch_scan_n(const DeltaParams& p, int n_seq, cudaStream_t st) {
     static bool done[64] = {};
     using R = Record<DKP>;
     const int stages = scan_stages<DKP>(p.some);
-    if (allow_smem(delta_scan_kernel<DKP, NC>, static_cast<size_t>(R::kStages) * R::kStageBytes, done) != cudaSuccess) return TBL_ERR_CUDA;
+    if (allow_smem(delta_scan_kernel<DKP, NC, OWN>, static_cast<size_t>(R::kStages) * R::kStageBytes, done) != cudaSuccess) return TBL_ERR_CUDA;
     const dim3 grid(ceil_div(p.dim, kScanLanes * NC), p.heads, n_seq);
-    const long long units = static_cast<long long>(n_seq) * p.heads * ((p.some + 1) / 2);
-    if (launch_dependent(delta_records_kernel<DKP>, dim3(ceil_div(units, 8)), dim3(256), 0, st, p, n_seq) != cudaSuccess) return TBL_ERR_CUDA;
-    return launch_dependent(delta_scan_kernel<DKP, NC>, grid, dim3(kScanThreads), static_cast<size_t>(stages) * R::kStageBytes, st, p, stages) == cudaSuccess
-               ? TBL_OK : TBL_ERR_CUDA;
+    if (!OWN) {
+        const long long units = static_cast<long long>(n_seq) * p.heads * ((p.some + 1) / 2);
+        if (launch_dependent(delta_records_kernel<DKP>, dim3(ceil_div(units, 8)), dim3(256), 0, st, p, n_seq) != cudaSuccess) return TBL_ERR_CUDA;
+    }
+    return launch_dependent(delta_scan_kernel<DKP, NC, OWN>, grid, dim3(scan_threads(DKP, NC, OWN)), static_cast<size_t>(stages) * R::kStageBytes, st, p,
+                            stages) == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 
 template <int DKP>
@@ -628,14 +653,20 @@ int launch_scan_d(const DeltaParams& p, int n_seq, cudaStream_t st) {
     // Narrow blocks of columns take less time a round (2000 tokens of 128 channels by 32, 16 and 8 columns: 8 heads 463, 364
     // and 305 us, in one wave each), a second wave of CTAs as long again (16 heads 480, 380 and 580; 32 heads 547, 766 and
     // 1159), and two to an SM a fifth longer than one.
-    const int room = scan_room<DKP>(p.some);
+    constexpr int room = scan_room(DKP);
     auto cost = [&](int cols, int us) {
         const long long ctas = static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq;
         return (ctas > kNumSm && room > kNumSm ? 6 : 5) * us * ((ctas + room - 1) / room);
     };
     const long long wide = cost(32, 480), half = cost(16, 380), narrow = cost(8, 305);
-    if (narrow <= half && narrow <= wide) return launch_scan_n<DKP, 1>(p, n_seq, st);
-    return half <= wide ? launch_scan_n<DKP, 2>(p, n_seq, st) : launch_scan_n<DKP, 4>(p, n_seq, st);
+    const int cols = narrow <= half && narrow <= wide ? 8 : (half <= wide ? 16 : 32);
+    // Records made in place take no launch of their own and no way through memory, but are made once per block of columns: 16
+    // heads of 128, 2, 16, 28 and 33 tokens 8.9, 15.5, 17.3 and 19.0 us, from memory 10.8, 18.5, 19.7 and 18.1; in more than one wave
+    // (8 such sequences, 16 tokens) 35.3 and 27.1.
+    const bool own = p.n_tok <= kOwnTokens && static_cast<long long>(ceil_div(p.dim, cols)) * p.heads * n_seq <= kNumSm;
+    if (cols == 8) return own ? launch_scan_n<DKP, 1, true>(p, n_seq, st) : launch_scan_n<DKP, 1, false>(p, n_seq, st);
+    if (cols == 16) return own ? launch_scan_n<DKP, 2, true>(p, n_seq, st) : launch_scan_n<DKP, 2, false>(p, n_seq, st);
+    return own ? launch_scan_n<DKP, 4, true>(p, n_seq, st) : launch_scan_n<DKP, 4, false>(p, n_seq, st);
 }
 
 template <typename T>
@@ -654,7 +685,7 @@ int launch_scan(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
     // idle, pieces of enough sequences side by side: a scan takes as long by itself (4 sequences of 1100 tokens, 8 heads of
     // 128, one after the other: 659 us).
     const int rounds = (p.n_tok + 1) / 2, most = max_rounds(p.heads, p.dim);
-    const int room = static_cast<int>(scan_room(p.dim, p.n_tok) / (static_cast<long long>(ceil_div(p.dim, 32)) * p.heads)), side = room < 1 ? 1 : room;
+    const int room = static_cast<int>(scan_room(padded_dim(p.dim)) / (static_cast<long long>(ceil_div(p.dim, 32)) * p.heads)), side = room < 1 ? 1 : room;
     int group = most / rounds, piece = p.n_tok;
     if (group >= n_seq) {
         group = n_seq;

@@ -438,9 +438,12 @@ def test_delta_scan_in_pieces_and_groups(cuda, stack_lib, seqs, heads, dim, n):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
-@pytest.mark.parametrize("seqs,heads,dim,n,scans", [(10, 2, 128, 1800, 2), (7, 1, 256, 4000, 2), (5, 40, 128, 300, 3), (32, 1, 64, 700, 1), (4, 8, 128, 1100, 1)])
+@pytest.mark.parametrize("seqs,heads,dim,n,scans", [(10, 2, 128, 1800, 2), (7, 1, 256, 4000, 2), (5, 40, 128, 300, 3), (32, 1, 64, 700, 1), (4, 8, 128, 1100, 1),
+                                                     (40, 8, 128, 17, 1), (12, 16, 128, 32, 1), (6, 36, 128, 24, 1), (30, 16, 64, 31, 1), (200, 20, 40, 5, 1),
+                                                     (20, 3, 200, 9, 1), (3, 16, 256, 11, 1), (64, 5, 22, 6, 1)])
 def test_delta_sequences_side_by_side(cuda, stack_lib, seqs, heads, dim, n, scans):
-    """Sequences of a batch come out as they do alone, bit for bit, whole or in pieces, and are not scanned one after the other."""
+    """Sequences of a batch come out as they do alone, bit for bit, whole or in pieces, and are not scanned one after the other.  Up to 32
+    tokens the scan of one sequence makes its records itself."""
     torch, rng = cuda, np.random.default_rng(n)
     torch.manual_seed(n)
     b = Buf(torch)
