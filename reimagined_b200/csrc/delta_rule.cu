@@ -125,7 +125,8 @@ __device__ __forceinline__ void make_record(const DeltaParams& p, int head, size
     using R = Record<DKP>;
     constexpr int NI = (DKP + 127) / 128;      // groups of four channels per lane
     const int lane = threadIdx.x & 31, dim = p.dim, HD = p.heads * dim;
-    const bool vec = ((dim | p.ld) & 3) == 0;          // every row and head starts on 16 bytes
+    // every row and head starts on 16 bytes
+    const bool vec = ((dim | p.ld) & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.w0)) & 15) == 0;
     auto load4 = [&](const float* base, int c, bool live) {
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (!live || c >= dim) return v;

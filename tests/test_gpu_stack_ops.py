@@ -467,6 +467,27 @@ def test_delta_sequences_side_by_side(cuda, stack_lib, seqs, heads, dim, n, scan
     assert bool(torch.isfinite(out).all()) and stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+@pytest.mark.parametrize("n", [9, 35])
+def test_delta_scan_of_unaligned_projections(cuda, stack_lib, n):
+    """Projections and decay biases that start on 4 bytes: the same as those that start on 16."""
+    torch, rng = cuda, np.random.default_rng(n)
+    b = Buf(torch)
+    m, _, w0, _ = delta_mixer(torch, b, 2, 32, 4, rng)
+    proj, results = 0.8 * torch.randn(n * (5 * 64 + 4), device="cuda"), []
+    biases = torch.cat([torch.zeros(1), torch.as_tensor(w0).float()]).cuda()
+    for shift in (0, 1):
+        at = torch.cat([torch.zeros(shift, device="cuda"), proj])
+        m.decay_up.bias = biases[1:].data_ptr() if shift else b.f32(w0)
+        assert (at[shift:].data_ptr() % 16 != 0) == bool(shift)
+        states, out = torch.zeros((1, 2, 32, 32), device="cuda"), torch.full((n, 64), float("nan"), device="cuda")
+        size = stack_lib.tbl_delta_workspace_bytes(C.byref(m), 0, n)
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        assert stack_lib.tbl_delta_forward(C.byref(m), 0, DELTA_SCAN, 1e-3, at[shift:].data_ptr(), states.data_ptr(), b.i32([0]), 1, n, out.data_ptr(),
+                                           ws.data_ptr(), size, stream(torch)) == 0
+        results.append(torch.cat([out.flatten(), states.flatten()]))
+    assert torch.equal(*results)
+
+
 def test_delta_scan_refuses_more_sequences_than_a_grid_has(cuda, stack_lib):
     torch, rng = cuda, np.random.default_rng(0)
     b = Buf(torch)
