@@ -244,8 +244,11 @@ int launch_depth_norm_streams(const DepthNorm& p, cudaStream_t st) {
 int launch_depth_norm(int precision, const DepthNorm& p, cudaStream_t st) {
     static_assert(TBL_MAX_STREAMS == 8, "the cases above");
     if (p.rows <= 0) return TBL_OK;
-    // a cluster per row as long as that is a few CTAs to an SM: 64 rows of 4096 by 64 CTAs took 8 to 14 us, by 512 CTAs 4 to 6
-    const bool spread = p.rows <= 64 && p.width >= 512;
+    // A cluster per row up to 32 rows, and up to 64 where its exchange of the sums costs less than the row by itself (64 rows, one array, by one
+    // CTA and by eight: 512 wide 2.2 and 4.3 us, 2048 3.8 and 4.6, 4096 6.1 and 5.0, 8192 10.5 and 5.7).  Dynamic Tanh has no sums
+    // to exchange (48 rows, two streams: 512 wide 2.3 and 2.3, 2048 4.1 and 2.6; 64 rows: 512 wide 2.3 and 2.6, 2048 4.2 and 2.8).
+    const bool sums = p.norm_kind == TBL_NORM_RMS;
+    const bool spread = p.width >= 512 && (p.rows <= 32 || (p.rows <= 64 && p.width >= (sums ? 3072 : (p.rows <= 48 ? 512 : 1536))));
     if (precision == TBL_BF16) return spread ? launch_depth_norm_streams<bf16, 8>(p, st) : launch_depth_norm_streams<bf16, 1>(p, st);
     return spread ? launch_depth_norm_streams<float, 8>(p, st) : launch_depth_norm_streams<float, 1>(p, st);
 }

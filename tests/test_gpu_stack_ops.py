@@ -343,7 +343,7 @@ def test_mixer_weights_made_by_the_kernel_before(cuda, stack_lib, precision, seq
 
 # ---- norm and depth average -----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("rows,width,count", [(1, 512, 1), (3, 1000, 12), (40, 90, 5), (2, 4100, 19), (33, 516, 9)])
+@pytest.mark.parametrize("rows,width,count", [(1, 512, 1), (3, 1000, 12), (40, 90, 5), (2, 4100, 19), (33, 516, 9), (33, 3072, 2), (64, 4100, 3), (65, 3074, 1), (64, 3070, 2)])
 def test_depth_norm(cuda, stack_lib, precision, rows, width, count):
     torch, rng = cuda, np.random.default_rng(width)
     b = Buf(torch)
@@ -675,7 +675,7 @@ def test_latent_attention_reports_a_full_cache(cuda, stack_lib):
 
 # ---- residual streams and Dynamic Tanh ------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("rows,width,streams", [(1, 512, 2), (3, 1000, 1), (40, 90, 3), (2, 4100, 4), (33, 516, 8), (5, 37, 5), (70, 64, 6), (32, 2048, 7)])
+@pytest.mark.parametrize("rows,width,streams", [(1, 512, 2), (3, 1000, 1), (40, 90, 3), (2, 4100, 4), (33, 516, 8), (5, 37, 5), (70, 64, 6), (32, 2048, 7), (64, 3076, 2), (48, 514, 2), (64, 1536, 3), (49, 1530, 4)])
 def test_stream_norm(cuda, stack_lib, precision, rows, width, streams):
     """Update, store, sum, next input and both norms; then rows picked out without a store."""
     torch, rng = cuda, np.random.default_rng(width)
