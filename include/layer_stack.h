@@ -10,7 +10,9 @@
  * and launch counter are declared there too (each library has its own copy of the latter two).
  *
  * Precision.  TBL_BF16: matrix-product operands (weights, normed rows, cached latents, queries) are bfloat16 with
- * fp32 accumulation.  TBL_F32: activations and caches are fp32 and every product is a plain fp32 FMA.  In both, the
+ * fp32 accumulation.  TBL_F32: activations and caches are fp32 and so is every product: a plain FMA, or in linear layers
+ * of more than four rows (where K and the row stride of W are multiples of 8) the sum of the exact products of three bf16
+ * pieces of x, which errs less than a chain of FMAs.  No number is rounded to fewer bits than fp32's.  In both, the
  * residual stream, norms, rotations, attention scores and weights, decays, step sizes, gates of the recurrence and
  * recurrent states are fp32.
  *
@@ -167,7 +169,8 @@ int tbl_stack_step(const tbl_stack_model* model, int precision, int slots, int c
  * result of earlier work on the stream, the weights too. */
 
 /* out[m, :] = W x[m, :] + b [+ residual[m, :]], fp32 out (ld = outputs of the view).  route: 0 the kernel the step
- * would take, 1 the SIMT kernel, 2 the GEMV, 3 the tcgen05 GEMM (bf16 only), 4 the row-streaming kernel (bf16 only);
+ * would take (fp32 rows beyond the GEMV's: the tcgen05 kernel with x in three pieces, or the SIMT kernel; it has no
+ * number of its own), 1 the SIMT kernel, 2 the GEMV, 3 the tcgen05 GEMM (bf16 only), 4 the row-streaming kernel (bf16 only);
  * TBL_ERR_SHAPE when the route does not take the shape. */
 int tbl_dense_forward(const tbl_dense_view* view, int precision, int route, const void* x_dev, int ldx, int rows,
                       const float* residual_dev, float* out_dev, void* stream);

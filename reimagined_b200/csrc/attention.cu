@@ -261,9 +261,11 @@ int pick_splits(const tbl_attention_mixer& m, int route, int n_seq, int n_tok, i
     if (s > tokens) s = tokens;
     // a cluster's worth is enough when that keeps most of the SMs busy, or leaves a CTA little to read
     if (route == kStream && s > kClusterSplits && (units * kClusterSplits >= kNumSm / 2 || tokens <= 8 * kClusterSplits)) s = kClusterSplits;
-    // Clusters of more than four that want nearly every place of two to an SM (264 for eight) wait for each other, and leave the linear
-    // layers around them no room: up to 4096 tokens four CTAs are faster there (8 sequences x 4 heads, 900 tokens: 234 us a step of
-    // four layers, now 214; 12 x 4, 800: 330 and 290; at 6000 tokens the same), with 28 units of eight they are not (202 and 214).
+    // Clusters of more than four that want nearly every place of two to an SM (clusters of eight find 264) wait for each other, and leave
+    // the linear layers around them no room: up to 4096 tokens four CTAs are faster there in a step (four layers: 32 units of 900 tokens
+    // 239 and 217 us, of 3900 306 and 299; 48 units of 900 333 and 297; at 6000 tokens the same), although not by themselves (32 units
+    // of 900 tokens 12.8 and 13.9 us, of 3900 22.5 and 30.3).  28 units of eight, 224 CTAs, leave room enough (202 us, by four 214); the
+    // line lies between those and the 256 of 32 units.
     if (route == kStream && s > 4 && s <= kClusterSplits && tokens <= 64 && units * s > 240) s = 4;
     return s < 1 ? 1 : (s > kMergeMaxSplits ? kMergeMaxSplits : static_cast<int>(s));
 }
