@@ -203,9 +203,10 @@ int launch_gemv_u(const DenseCall& c, cudaStream_t st) {
 
 // One or two rows per warp are bound by the bytes on their way: 6144 -> 2048 at one fp32 row takes 18.4 us with one step a batch
 // and 6.4 with eight.  One step it is where there is no second one and at most a block to an SM (256 -> 256: 1.8 and 1.9 us at
-// two rows), and of two rows per warp where two steps' registers mean another wave of blocks: each wave takes as long as it has
+// two rows), and of two rows per warp and two to four fp32 rows where two steps' registers mean another wave of blocks: each wave takes as long as it has
 // blocks to an SM (2048 -> 10304, 644 blocks: three rows 16.2 us in one wave of five and 18.9 in two of three, four rows 24.6 in two
-// of four and 22.3 in two of three).
+// of four and 22.3 in two of three).  At one row two waves are as fast by themselves (gated 2048 -> 6144 12.5 and 12.8 us, by one
+// and two steps) and faster in a step, where the first loads are under way before it starts (width 2048: 231 and 228 us).
 template <typename T, int M, int R>
 int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
     const long long ctas = ceil_div(c.pair_cols ? ceil_div(c.pair_cols, R / 2 > 0 ? R / 2 : 1) : ceil_div(c.N, R), kGemvWarps);
@@ -214,7 +215,7 @@ int launch_gemv_r(const DenseCall& c, cudaStream_t st) {
     if constexpr (R == 2) {
         const int fit = static_cast<int>(227 * 1024 / (sizeof(float) * M * c.K + 1024));     // blocks to an SM by shared memory, and by registers
         auto cost = [&](int regs) { const long long n = fit < regs ? fit : regs; return n * ((ctas + n * kNumSm - 1) / (n * kNumSm)); };
-        if (c.K >= 512 && cost(M <= 2 ? 4 : 3) <= cost(M <= 2 ? 6 : (M == 3 ? 5 : 4))) return launch_gemv_u<T, M, 2, 2>(c, st);
+        if (c.K >= 512 && (M == 1 || cost(M <= 2 ? 4 : 3) <= cost(M <= 2 ? 6 : (M == 3 ? 5 : 4)))) return launch_gemv_u<T, M, 2, 2>(c, st);
     }
     return launch_gemv_u<T, M, R, 1>(c, st);
 }
