@@ -20,7 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBRARIES = {
     "ternary": (os.path.join(HERE, "libternary_b200.so"),
                 ["runtime.cu", "api.cu", "quantize.cu", "gemv_stream.cu", "gemv_generic.cu", "gemv_strip.cu",
-                 "gemv_chain.cu", "gemm_tcgen05.cu", "gemm_widen.cu", "moe.cu", "glue.cu", "decode.cu", "packer.cpp",
+                 "gemv_chain.cu", "gemm_tcgen05.cu", "gemm_widen.cu", "moe.cu", "glue.cu", "decode.cu", "decode_cluster.cu", "packer.cpp",
                  "edge_pack.cpp"]),
     "stack": (os.path.join(HERE, "libstack_b200.so"),
               ["runtime.cu", "stack.cu", "stack_glue.cu", "dense.cu", "dense_rows.cu", "dense_tcgen05.cu", "dense_split.cu", "delta_rule.cu",

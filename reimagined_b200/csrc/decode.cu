@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "decode_cluster.cuh"
 #include "kernels.cuh"
 
 namespace tbl {
@@ -1085,7 +1086,20 @@ int tbl_decode_step(const tbl_decode_model* model, int batch, int capacity, void
         return pre;
     };
     int cur = 0;
-    for (int i = 0; i < m.n_blocks; ++i) {
+    // All blocks in one launch where the cluster kernel takes the model; the loop below is the general route.
+    ClusterShape shape;
+    bool in_clusters = decode_cluster_shape(m, B, capacity, &shape);
+    for (int i = 0; i < m.n_blocks && in_clusters; ++i)
+        if (m.blocks[i].hybrid) in_clusters = attention_smem_bytes(m.blocks[i].attn.head_dim, capacity) <= 200 * 1024;   // refused below
+    if (in_clusters) {
+        ClusterBlockState cs[TBL_MAX_DECODE_BLOCKS];
+        for (int i = 0; i < m.n_blocks; ++i) cs[i] = ClusterBlockState{state.block[i].ring, state.block[i].ssm, state.block[i].k_cache, state.block[i].v_cache};
+        if (launch_decode_cluster(m, shape, B, capacity, cs, state.positions, token_ids_dev, S.hidden[0], hidden_trace_dev, status, st) != cudaSuccess)
+            return TBL_ERR_CUDA;
+        pend = Pending{S.hidden[0], nullptr, nullptr, nullptr, nullptr, nullptr};
+        cur = 1;
+    }
+    for (int i = 0; i < m.n_blocks && !in_clusters; ++i) {
         const tbl_decode_block& b = m.blocks[i];
         const tbl_mamba_block& mm = b.mamba;
         if (mm.d_inner > 16 * 1024) return TBL_ERR_SHAPE;
@@ -1231,6 +1245,7 @@ int tbl_decode_step(const tbl_decode_model* model, int batch, int capacity, void
             return rc;
         if ((rc = linear(m.head, S.core, logits_dev)) != TBL_OK) return rc;
     }
+    if (in_clusters) return TBL_OK;
     advance_positions_kernel<<<(B + 127) / 128, 128, 0, st>>>(state.positions, B);
     return launched();
 }
