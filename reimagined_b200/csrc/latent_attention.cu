@@ -75,47 +75,66 @@ __global__ void __launch_bounds__(kPrepThreads) latent_prep_kernel(const LatentP
     }
 }
 
-// One CTA per (row, head): q' [R] = sum_d q[d] W_uk[head, d, :], then the rotated part of q.
-template <typename T>
-__global__ void __launch_bounds__(128) latent_absorb_kernel(const LatentParams p) {
-    extern __shared__ float q[];                  // [d + rd]
+// q' [R] = sum_d q[d] W_uk[head, d, :], then the rotated part of q.  One CTA per RT rows, head and 64 of the R columns: a lane takes two of them, the
+// four warps a fourth of the sum each.  Bound by latency for one row: as one CTA per head (16 CTAs, eight trips to memory one after the other) 34.6 us
+// for 16 heads of 128 x 512 (2 MB), now every thread has its 32 loads in flight at once.  Eight rows share the weights: 251 rows 79 us before.
+constexpr int kAbsorbCols = 64;
+template <typename T, int RT>
+__global__ void __launch_bounds__(128) latent_absorb_kernel(const LatentParams p, int rows) {
+    extern __shared__ float q[];                  // [d][RT]
+    __shared__ float part[4][RT][kAbsorbCols];
     pdl_launch_dependents();
-    const int row = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, n = p.d + p.rd;
+    const int row0 = blockIdx.x * RT, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n = p.d + p.rd, R = min(RT, rows - row0);
     pdl_wait();
-    const int slot = p.slots[row / p.n_tok];
-    const int pos = min(max(p.positions[slot] + row % p.n_tok, 0), p.rope_positions - 1);
-    const float* qr = p.q + (static_cast<size_t>(row) * p.H + head) * n;
-    for (int e = tid; e < n; e += 128) q[e] = qr[e];
+    for (int i = tid; i < RT * p.d; i += 128) {
+        const int r = i / p.d, k = i - r * p.d;
+        q[k * RT + r] = r < R ? p.q[(static_cast<size_t>(row0 + r) * p.H + head) * n + k] : 0.0f;
+    }
     __syncthreads();
-    T* out = static_cast<T*>(p.qa) + (static_cast<size_t>(row) * p.H + head) * p.cw;
     const bf16* w = p.uk + static_cast<size_t>(head) * p.d * p.R;
+    const int e = blockIdx.z * kAbsorbCols + 2 * lane, per = (p.d + 3) >> 2, k0 = warp * per, k1 = min(p.d, k0 + per);
+    float a[RT], b[RT];
+#pragma unroll
+    for (int r = 0; r < RT; ++r) a[r] = b[r] = 0.0f;
+    auto add = [&](int k, float x, float y) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r) { a[r] = fmaf(q[k * RT + r], x, a[r]); b[r] = fmaf(q[k * RT + r], y, b[r]); }
+    };
     if ((p.R & 1) == 0) {
-        for (int e = 2 * tid; e < p.R; e += 256) {
-            float a = 0.0f, b = 0.0f;
-#pragma unroll 16
-            for (int k = 0; k < p.d; ++k) {
+        if (e < p.R) {
+#pragma unroll 32
+            for (int k = k0; k < k1; ++k) {
                 const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(w + static_cast<size_t>(k) * p.R + e));
-                a = fmaf(q[k], bf_lo(v), a);
-                b = fmaf(q[k], bf_hi(v), b);
+                add(k, bf_lo(v), bf_hi(v));
             }
-            out[e] = from_f<T>(a);
-            out[e + 1] = from_f<T>(b);
         }
     } else {
-        for (int e = tid; e < p.R; e += 128) {
-            float a = 0.0f;
-            for (int k = 0; k < p.d; ++k) a = fmaf(q[k], to_f(w[static_cast<size_t>(k) * p.R + e]), a);
-            out[e] = from_f<T>(a);
+        for (int k = k0; k < k1; ++k) {
+            const bf16* v = w + static_cast<size_t>(k) * p.R + e;
+            add(k, e < p.R ? to_f(v[0]) : 0.0f, e + 1 < p.R ? to_f(v[1]) : 0.0f);
         }
     }
-    const int half = p.rd / 2;
-    for (int i = tid; i < half; i += 128) {
-        const float cv = __ldg(p.rope_cos + static_cast<size_t>(pos) * half + i), sv = __ldg(p.rope_sin + static_cast<size_t>(pos) * half + i);
-        const float u = q[p.d + i], v = q[p.d + half + i];
-        out[p.R + i] = from_f<T>(u * cv - v * sv);
-        out[p.R + half + i] = from_f<T>(v * cv + u * sv);
+#pragma unroll
+    for (int r = 0; r < RT; ++r) *reinterpret_cast<float2*>(&part[warp][r][2 * lane]) = make_float2(a[r], b[r]);
+    __syncthreads();
+    T* out = static_cast<T*>(p.qa) + (static_cast<size_t>(row0) * p.H + head) * p.cw;
+    const size_t next = static_cast<size_t>(p.H) * p.cw;          // from row to row
+    for (int i = tid; i < R * kAbsorbCols; i += 128) {
+        const int r = i / kAbsorbCols, c = i % kAbsorbCols, col = blockIdx.z * kAbsorbCols + c;
+        if (col < p.R) out[r * next + col] = from_f<T>((part[0][r][c] + part[1][r][c]) + (part[2][r][c] + part[3][r][c]));
     }
-    for (int e = p.R + p.rd + tid; e < p.cw; e += 128) out[e] = from_f<T>(0.0f);
+    if (blockIdx.z) return;
+    const int half = p.rd / 2, tail = p.cw - p.R - p.rd;
+    for (int i = tid; i < R * half; i += 128) {
+        const int r = i / half, k = i - r * half, row = row0 + r;
+        const int pos = min(max(p.positions[p.slots[row / p.n_tok]] + row % p.n_tok, 0), p.rope_positions - 1);
+        const float cv = __ldg(p.rope_cos + static_cast<size_t>(pos) * half + k), sv = __ldg(p.rope_sin + static_cast<size_t>(pos) * half + k);
+        const float* rot = p.q + (static_cast<size_t>(row) * p.H + head) * n + p.d;
+        const float u = rot[k], v = rot[half + k];
+        out[r * next + p.R + k] = from_f<T>(u * cv - v * sv);
+        out[r * next + p.R + half + k] = from_f<T>(v * cv + u * sv);
+    }
+    for (int i = tid; i < R * tail; i += 128) out[i / tail * next + p.R + p.rd + i % tail] = from_f<T>(0.0f);
 }
 
 // One CTA of four warps per (row, head, split); a warp takes every fourth token pair of the split, lanes share the
@@ -181,54 +200,90 @@ __global__ void __launch_bounds__(32 * kSimtWarps) latent_simt_kernel(const Late
     if (tid == 0) { p.part_m[unit] = mt; p.part_l[unit] = lt; }
 }
 
-// One CTA per (row, head): merge, W_uv, gate.
-template <typename T>
-__global__ void __launch_bounds__(256) latent_value_kernel(const LatentParams p) {
-    extern __shared__ float sm[];                // [R] latent | [splits] factors
+// Merge, W_uv, gate.  One CTA per RT rows, head and 32 of the vdim outputs, four outputs a warp, whose weights are requested together: as one CTA per
+// head, a warp's sixteen outputs one after the other, 21 us for one row of 16 heads of 128 x 512, and 139 us for 251.
+constexpr int kValueRows = 32, kValueEach = kValueRows / 8;
+template <typename T, int RT>
+__global__ void __launch_bounds__(256) latent_value_kernel(const LatentParams p, int rows) {
+    extern __shared__ float sm[];                // [RT][R] latents | [RT][splits] factors
     float* lat = sm;
-    float* fac = sm + p.R;
-    __shared__ float total_s;
+    float* fac = sm + RT * p.R;
+    __shared__ float total_s[RT];
     pdl_launch_dependents();
-    const int row = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row0 = blockIdx.x * RT, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, R = min(RT, rows - row0);
     pdl_wait();
-    const size_t unit = (static_cast<size_t>(row) * p.H + head) * p.splits;
-    if (warp == 0) {
+    auto unit = [&](int r) { return (static_cast<size_t>(row0 + r) * p.H + head) * p.splits; };
+    static_assert(RT <= 8, "a warp a row");
+    if (warp < R) {
+        const float *pm = p.part_m + unit(warp), *pl = p.part_l + unit(warp);
         float m = -INFINITY, l = 0.0f;
-        for (int s = lane; s < p.splits; s += 32) m = fmaxf(m, p.part_m[unit + s]);
+        for (int s = lane; s < p.splits; s += 32) m = fmaxf(m, pm[s]);
         m = warp_max(m);
         for (int s = lane; s < p.splits; s += 32) {
-            const float ms = p.part_m[unit + s], f = ms == -INFINITY ? 0.0f : expf(ms - m);
-            fac[s] = f;
-            l = fmaf(p.part_l[unit + s], f, l);
+            const float ms = pm[s], f = ms == -INFINITY ? 0.0f : expf(ms - m);
+            fac[warp * p.splits + s] = f;
+            l = fmaf(pl[s], f, l);
         }
         l = warp_sum(l);
-        if (lane == 0) total_s = 1.0f / l;
+        if (lane == 0) total_s[warp] = 1.0f / l;
     }
     __syncthreads();
-    for (int e = tid; e < p.R; e += 256) {
+    for (int i = tid; i < RT * p.R; i += 256) {
+        const int r = i / p.R, e = i - r * p.R;
         float v = 0.0f;
+        if (r < R) {
+            const float* o = p.part_o + unit(r) * p.R + e;
 #pragma unroll 4
-        for (int s = 0; s < p.splits; ++s) v = fmaf(p.part_o[(unit + s) * p.R + e], fac[s], v);
-        lat[e] = v * total_s;
+            for (int s = 0; s < p.splits; ++s) v = fmaf(o[static_cast<size_t>(s) * p.R], fac[r * p.splits + s], v);
+            v *= total_s[r];
+        }
+        lat[i] = v;
     }
     __syncthreads();
-    const float* g = p.proj + static_cast<size_t>(row) * p.ld + p.q_rank + p.R + p.rd + head * p.vd;
-    T* out = static_cast<T*>(p.out) + static_cast<size_t>(row) * p.H * p.vd + head * p.vd;
-    for (int v = warp; v < p.vd; v += 8) {
-        const bf16* w = p.uv + static_cast<size_t>(head * p.vd + v) * p.R;
-        float a = 0.0f;
-        if ((p.R & 7) == 0) {
-            for (int e = lane * 8; e < p.R; e += 256) {
-                const uint4 x = __ldg(reinterpret_cast<const uint4*>(w + e));
-                const float4 s = *reinterpret_cast<const float4*>(lat + e), t = *reinterpret_cast<const float4*>(lat + e + 4);
-                a = fmaf(bf_lo(x.x), s.x, a); a = fmaf(bf_hi(x.x), s.y, a); a = fmaf(bf_lo(x.y), s.z, a); a = fmaf(bf_hi(x.y), s.w, a);
-                a = fmaf(bf_lo(x.z), t.x, a); a = fmaf(bf_hi(x.z), t.y, a); a = fmaf(bf_lo(x.w), t.z, a); a = fmaf(bf_hi(x.w), t.w, a);
+    const int v0 = blockIdx.z * kValueRows + warp * kValueEach;
+    const bf16* w = p.uv + (static_cast<size_t>(head) * p.vd + v0) * p.R;
+    float a[kValueEach][RT];
+#pragma unroll
+    for (int j = 0; j < kValueEach; ++j)
+#pragma unroll
+        for (int r = 0; r < RT; ++r) a[j][r] = 0.0f;
+    if ((p.R & 7) == 0) {
+#pragma unroll 2
+        for (int e = lane * 8; e < p.R; e += 256) {
+            uint4 x[kValueEach];
+#pragma unroll
+            for (int j = 0; j < kValueEach; ++j) x[j] = v0 + j < p.vd ? __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(j) * p.R + e)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int r = 0; r < RT; ++r) {
+                const float4 s = *reinterpret_cast<const float4*>(lat + r * p.R + e), t = *reinterpret_cast<const float4*>(lat + r * p.R + e + 4);
+#pragma unroll
+                for (int j = 0; j < kValueEach; ++j) {
+                    float& b = a[j][r];
+                    b = fmaf(bf_lo(x[j].x), s.x, b); b = fmaf(bf_hi(x[j].x), s.y, b); b = fmaf(bf_lo(x[j].y), s.z, b); b = fmaf(bf_hi(x[j].y), s.w, b);
+                    b = fmaf(bf_lo(x[j].z), t.x, b); b = fmaf(bf_hi(x[j].z), t.y, b); b = fmaf(bf_lo(x[j].w), t.z, b); b = fmaf(bf_hi(x[j].w), t.w, b);
+                }
             }
-        } else {
-            for (int e = lane; e < p.R; e += 32) a = fmaf(to_f(w[e]), lat[e], a);
         }
-        a = warp_sum(a);
-        if (lane == 0) out[v] = from_f<T>(a * sigmoid_f(g[v]));
+    } else {
+        for (int e = lane; e < p.R; e += 32)
+#pragma unroll
+            for (int j = 0; j < kValueEach; ++j) {
+                const float x = v0 + j < p.vd ? to_f(w[static_cast<size_t>(j) * p.R + e]) : 0.0f;
+#pragma unroll
+                for (int r = 0; r < RT; ++r) a[j][r] = fmaf(x, lat[r * p.R + e], a[j][r]);
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < kValueEach; ++j) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+            const float v = warp_sum(a[j][r]);
+            if (lane == j * RT + r && r < R && v0 + j < p.vd) {
+                const size_t row = row0 + r;
+                const float g = p.proj[row * p.ld + p.q_rank + p.R + p.rd + head * p.vd + v0 + j];
+                static_cast<T*>(p.out)[row * p.H * p.vd + head * p.vd + v0 + j] = from_f<T>(v * sigmoid_f(g));
+            }
+        }
     }
 }
 
@@ -309,11 +364,19 @@ int run(const tbl_latent_mixer& m, LatentParams p, const Plan& w, int precision,
         return launch_latent_expanded(m, p, n_seq, st);
     }
     if (w.route == kCacheTensor) return launch_latent_tensor(p, rows, st);
-    if (launch_dependent(latent_absorb_kernel<T>, dim3(rows, p.H), dim3(128), sizeof(float) * (p.d + p.rd), st, p) != cudaSuccess)
+    // several rows share the weights, where their queries and latents fit the shared memory that needs no asking for
+    constexpr int kTile = 8;
+    const bool tiled = rows > 4 && p.d <= 1024 && sizeof(float) * kTile * (p.R + p.splits) <= 40 * 1024;
+    const int tiles = tiled ? ceil_div(rows, kTile) : rows, per = tiled ? kTile : 1;
+    const dim3 absorb(tiles, p.H, ceil_div(p.R, kAbsorbCols)), value(tiles, p.H, ceil_div(p.vd, kValueRows));
+    const size_t absorb_smem = sizeof(float) * per * p.d, value_smem = sizeof(float) * per * (p.R + p.splits);
+    if ((tiled ? launch_dependent(latent_absorb_kernel<T, kTile>, absorb, dim3(128), absorb_smem, st, p, rows)
+               : launch_dependent(latent_absorb_kernel<T, 1>, absorb, dim3(128), absorb_smem, st, p, rows)) != cudaSuccess)
         return TBL_ERR_CUDA;
     rc = launch_simt<T>(p, rows, st);
     if (rc != TBL_OK) return rc;
-    return launch_dependent(latent_value_kernel<T>, dim3(rows, p.H), dim3(256), sizeof(float) * (p.R + p.splits), st, p) == cudaSuccess
+    return (tiled ? launch_dependent(latent_value_kernel<T, kTile>, value, dim3(256), value_smem, st, p, rows)
+                  : launch_dependent(latent_value_kernel<T, 1>, value, dim3(256), value_smem, st, p, rows)) == cudaSuccess
                ? TBL_OK : TBL_ERR_CUDA;
 }
 
