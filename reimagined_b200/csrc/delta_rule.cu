@@ -32,6 +32,22 @@ __device__ __forceinline__ float sum8lanes(float v) {
     return v;
 }
 
+// The sums of eight columns over the LANES lanes that hold them, each in the order of sum8lanes: three exchanges that halve the number of values, then
+// plain ones (nine for 32 lanes, where every column by itself takes five).  Lane l has the sum of column l % 8, bits reversed.
+__device__ __forceinline__ constexpr int bits3(int n) { return (n & 1) << 2 | (n & 2) | (n & 4) >> 2; }
+template <int LANES>
+__device__ __forceinline__ float sum_columns8(const float* v, int lane) {
+    float a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = (lane & 1 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, lane & 1 ? v[i] : v[i + 4], 1);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) b[i] = (lane & 2 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, lane & 2 ? a[i] : a[i + 2], 2);
+    float r = (lane & 4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[0] : b[1], 4);
+#pragma unroll
+    for (int o = 8; o < LANES; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+}
+
 // Four keys of one column (key index c .. c+3, clipped at dim): state <-> registers.
 __device__ __forceinline__ ulonglong2 load_state4(const float* col, int c, int dim) {
     if ((dim & 3) == 0) {
@@ -448,10 +464,11 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const DeltaParams p, int
 }
 
 // ---- one token ------------------------------------------------------------------------------------------------------
-// THREADS / 8 column groups; a thread's columns are its group + i * THREADS / 8, taken NCP at a time.
-template <typename T, int DKP, int THREADS, int NCP, bool FUSED>
-__global__ void __launch_bounds__(THREADS, DKP == 128 ? 2 : 1) delta_step_kernel(const DeltaParams p) {
-    constexpr int G = DKP / 32, GROUPS = THREADS / 8, PASSES = DKP / (GROUPS * NCP);
+// LANES lanes share a column, NCP columns of a group of lanes are in flight; a group's columns are its number + i * THREADS / LANES.
+template <typename T, int DKP, int THREADS, int LANES, int NCP, int BLOCKS, bool FUSED>
+__global__ void __launch_bounds__(THREADS, BLOCKS) delta_step_kernel(const DeltaParams p) {
+    constexpr int G = DKP / (4 * LANES), GROUPS = THREADS / LANES, PASSES = DKP / (GROUPS * NCP);
+    static_assert(NCP % 8 == 0 || LANES == 8, "columns are added eight at a time");
     static_assert(PASSES >= 1 && PASSES * GROUPS * NCP == DKP, "columns of a head");
     __shared__ __align__(16) float su[DKP], sw[DKP], sau[DKP], sk[DKP], sr[DKP], sv[DKP], so[DKP], part[FUSED ? THREADS : 1];
     extern __shared__ float st_tanh[];         // [rank]
@@ -463,7 +480,7 @@ __global__ void __launch_bounds__(THREADS, DKP == 128 ? 2 : 1) delta_step_kernel
     for (int e = tid * 32; e < dim * dim; e += THREADS * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(st + e));
     pdl_wait();
     const float* pr = p.proj + static_cast<size_t>(row) * p.ld;
-    const int l8 = tid & 7, group = tid >> 3;
+    const int lg = tid & (LANES - 1), group = tid / LANES;
     ulonglong2 S[NCP][G];
     auto load_pass = [&](int ps) {
 #pragma unroll
@@ -471,7 +488,7 @@ __global__ void __launch_bounds__(THREADS, DKP == 128 ? 2 : 1) delta_step_kernel
             const int j = (ps * NCP + n) * GROUPS + group;
 #pragma unroll
             for (int g = 0; g < G; ++g)
-                S[n][g] = j < dim ? load_state4(st + static_cast<size_t>(j) * dim, 4 * (l8 + 8 * g), dim) : make_ulonglong2(0, 0);
+                S[n][g] = j < dim ? load_state4(st + static_cast<size_t>(j) * dim, 4 * (lg + LANES * g), dim) : make_ulonglong2(0, 0);
         }
     };
     // everything that depends on this step's projections is requested first, then the state
@@ -527,35 +544,59 @@ __global__ void __launch_bounds__(THREADS, DKP == 128 ? 2 : 1) delta_step_kernel
         sau[tid] = sigmoid_f(a_in) * u;
     }
     __syncthreads();
-    const ulonglong2 *qu = reinterpret_cast<const ulonglong2*>(su) + l8, *qw = reinterpret_cast<const ulonglong2*>(sw) + l8,
-                     *qa = reinterpret_cast<const ulonglong2*>(sau) + l8, *qk = reinterpret_cast<const ulonglong2*>(sk) + l8,
-                     *qr = reinterpret_cast<const ulonglong2*>(sr) + l8;
+    const ulonglong2 *qu = reinterpret_cast<const ulonglong2*>(su) + lg, *qw = reinterpret_cast<const ulonglong2*>(sw) + lg,
+                     *qa = reinterpret_cast<const ulonglong2*>(sau) + lg, *qk = reinterpret_cast<const ulonglong2*>(sk) + lg,
+                     *qr = reinterpret_cast<const ulonglong2*>(sr) + lg;
 #pragma unroll 1
     for (int ps = 0; ps < PASSES; ++ps) {
+        asm volatile("" ::: "memory");         // the head's vectors stay in shared memory, not in registers across the passes
         if (ps > 0) load_pass(ps);
-        pair2 m[NCP], vv[NCP];
+        float sums[NCP];
 #pragma unroll
         for (int n = 0; n < NCP; ++n) {
             pair2 d = 0, e = 0;
 #pragma unroll
-            for (int g = 0; g < G; ++g) { d = fma2(qu[8 * g].x, S[n][g].x, d); e = fma2(qu[8 * g].y, S[n][g].y, e); }
-            m[n] = dup2(-sum8lanes(sum2(add2(d, e))));
-            vv[n] = dup2(sv[(ps * NCP + n) * GROUPS + group]);
+            for (int g = 0; g < G; ++g) { d = fma2(qu[LANES * g].x, S[n][g].x, d); e = fma2(qu[LANES * g].y, S[n][g].y, e); }
+            sums[n] = sum2(add2(d, e));
+        }
+        if constexpr (NCP % 8 == 0) {
+#pragma unroll
+            for (int b = 0; b < NCP; b += 8) {
+                const float r = sum_columns8<LANES>(sums + b, lane);
+#pragma unroll
+                for (int n = 0; n < 8; ++n) sums[b + n] = __shfl_sync(0xffffffffu, r, bits3(n), LANES);
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < NCP; ++n) sums[n] = sum8lanes(sums[n]);
         }
 #pragma unroll
         for (int n = 0; n < NCP; ++n) {
             const int j = (ps * NCP + n) * GROUPS + group;
+            const pair2 m = dup2(-sums[n]), vv = dup2(sv[j]);
             pair2 o = 0, f = 0;
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                S[n][g].x = fma2(qw[8 * g].x, S[n][g].x, fma2(qa[8 * g].x, m[n], mul2(qk[8 * g].x, vv[n])));
-                S[n][g].y = fma2(qw[8 * g].y, S[n][g].y, fma2(qa[8 * g].y, m[n], mul2(qk[8 * g].y, vv[n])));
-                o = fma2(qr[8 * g].x, S[n][g].x, o);
-                f = fma2(qr[8 * g].y, S[n][g].y, f);
-                if (j < dim) store_state4(st + static_cast<size_t>(j) * dim, 4 * (l8 + 8 * g), dim, S[n][g]);
+                S[n][g].x = fma2(qw[LANES * g].x, S[n][g].x, fma2(qa[LANES * g].x, m, mul2(qk[LANES * g].x, vv)));
+                S[n][g].y = fma2(qw[LANES * g].y, S[n][g].y, fma2(qa[LANES * g].y, m, mul2(qk[LANES * g].y, vv)));
+                o = fma2(qr[LANES * g].x, S[n][g].x, o);
+                f = fma2(qr[LANES * g].y, S[n][g].y, f);
+                if (j < dim) store_state4(st + static_cast<size_t>(j) * dim, 4 * (lg + LANES * g), dim, S[n][g]);
             }
-            const float r = sum8lanes(sum2(add2(o, f)));
-            if (l8 == 0) so[j] = r;
+            sums[n] = sum2(add2(o, f));
+        }
+        if constexpr (NCP % 8 == 0) {
+#pragma unroll
+            for (int b = 0; b < NCP; b += 8) {
+                const float r = sum_columns8<LANES>(sums + b, lane);
+                if (lg < 8) so[(ps * NCP + b + bits3(lg)) * GROUPS + group] = r;
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < NCP; ++n) {
+                const float r = sum8lanes(sums[n]);
+                if (lg == 0) so[(ps * NCP + n) * GROUPS + group] = r;
+            }
         }
     }
     __syncthreads();
@@ -582,10 +623,10 @@ int decay_products(const tbl_delta_mixer& m, const DeltaParams& p, int precision
     return launch_dense(precision, kDenseAuto, c, st);
 }
 
-template <typename T, int DKP, int THREADS, int NCP>
+template <typename T, int DKP, int THREADS, int LANES, int NCP, int BLOCKS>
 cudaError_t launch_step_d(const DeltaParams& p, dim3 grid, cudaStream_t st) {
-    return p.z ? launch_dependent(delta_step_kernel<T, DKP, THREADS, NCP, false>, grid, dim3(THREADS), 0, st, p)
-               : launch_dependent(delta_step_kernel<T, DKP, THREADS, NCP, true>, grid, dim3(THREADS), sizeof(float) * p.rank, st, p);
+    return p.z ? launch_dependent(delta_step_kernel<T, DKP, THREADS, LANES, NCP, BLOCKS, false>, grid, dim3(THREADS), 0, st, p)
+               : launch_dependent(delta_step_kernel<T, DKP, THREADS, LANES, NCP, BLOCKS, true>, grid, dim3(THREADS), sizeof(float) * p.rank, st, p);
 }
 
 struct Workspace {
@@ -618,10 +659,16 @@ int launch_step(const tbl_delta_mixer& m, DeltaParams p, int precision, int n_se
         p.z = w.z;
     }
     cudaError_t e;
-    if (p.dim <= 32) e = launch_step_d<T, 32, 256, 1>(p, grid, st);
-    else if (p.dim <= 64) e = launch_step_d<T, 64, 256, 2>(p, grid, st);
-    else if (p.dim <= 128) e = launch_step_d<T, 128, 256, 4>(p, grid, st);
-    else e = launch_step_d<T, 256, 512, 1>(p, grid, st);
+    // Bound by the states' bytes once the heads fill the chip, by the chain through one head before that.  A few heads: all of a head's columns in flight
+    // at once (at 128: 8 lanes a column, two blocks an SM).  More heads than fit at once: fewer columns and registers a thread and more blocks, so that
+    // one block's sums and stores run under the others' loads.  us for heads x dim x sequences, with the decay products of 256 channels ahead
+    // (before | after): 32x128x64 70.8 | 57.3 (states alone 41), 32x100x64 60.5 | 49.6, 32x128x16 23.7 | 22.1, 32x64x64 28.9 | 22.5, 12x64x64 15.4 | 11.9;
+    // not below it: 32x128x4 11.3 | 14.9, 32x64x8 7.7 | 9.3.  Heads of 256 with a warp a column need no spills: 16x256x32 68.9 | 59.8, 8x256x1 15.1 | 13.0.
+    const long long heads = static_cast<long long>(p.heads) * n_seq;
+    if (p.dim <= 32) e = launch_step_d<T, 32, 256, 8, 1, 1>(p, grid, st);
+    else if (p.dim <= 64) e = heads > 4 * kNumSm ? launch_step_d<T, 64, 128, 8, 4, 6>(p, grid, st) : launch_step_d<T, 64, 256, 8, 2, 1>(p, grid, st);
+    else if (p.dim <= 128) e = heads > 2 * kNumSm ? launch_step_d<T, 128, 256, 8, 1, 4>(p, grid, st) : launch_step_d<T, 128, 256, 8, 4, 2>(p, grid, st);
+    else e = launch_step_d<T, 256, 512, 32, 8, 1>(p, grid, st);
     return e == cudaSuccess ? TBL_OK : TBL_ERR_CUDA;
 }
 

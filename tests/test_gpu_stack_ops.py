@@ -416,6 +416,27 @@ def test_delta_rule_across_scan_and_single_steps(cuda, stack_lib, precision, hea
     assert not states[1].any()                    # nobody touched the third slot
 
 
+@pytest.mark.parametrize("seqs,heads,dim", [(4, 74, 128), (4, 75, 128), (9, 33, 100), (8, 74, 64), (8, 75, 64), (25, 24, 33), (3, 200, 64), (2, 170, 97), (5, 2, 256),
+                                            (4, 3, 131)])
+def test_delta_single_steps_of_many_heads(cuda, stack_lib, seqs, heads, dim):
+    """One token of up to as many heads as fit the chip at once, and of more: other splits of a head over the threads."""
+    torch, rng = cuda, np.random.default_rng(dim)
+    b = Buf(torch)
+    m, w2, w0, norm = delta_mixer(torch, b, heads, dim, 8, rng)
+    states = torch.as_tensor(rng.standard_normal((seqs, heads, dim, dim)), dtype=torch.float32).cuda()
+    want_states = f64(states).transpose(0, 1, 3, 2).copy()
+    proj = (0.8 * rng.standard_normal((seqs, 5 * heads * dim + 8))).astype(np.float32)
+    pd, out = torch.as_tensor(proj).cuda(), torch.zeros((seqs, heads * dim), device="cuda")
+    size = stack_lib.tbl_delta_workspace_bytes(C.byref(m), 0, seqs)
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    assert stack_lib.tbl_delta_forward(C.byref(m), 0, DELTA_STEP, 1e-3, pd.data_ptr(), states.data_ptr(), b.i32(range(seqs)), seqs, 1, out.data_ptr(),
+                                       ws.data_ptr(), size, stream(torch)) == 0
+    for i in range(seqs):
+        want = delta_oracle(proj[i:i + 1].astype(np.float64), heads, dim, w2, w0, norm, 1e-3, want_states[i])
+        assert_close(f64(out)[i:i + 1], want, 2e-5, f"sequence {i}")
+    assert_close(f64(states).transpose(0, 1, 3, 2), want_states, 2e-5, "states")
+
+
 @pytest.mark.parametrize("seqs,heads,dim,n", [(1, 1, 12, 2050), (40, 1, 16, 53), (2, 50, 8, 17), (1, 50, 32, 9), (3, 1, 256, 16)])
 def test_delta_scan_in_pieces_and_groups(cuda, stack_lib, seqs, heads, dim, n):
     """More rounds than the scan takes at a time (one sequence in pieces, many in groups), and each width of a block of columns."""
