@@ -33,7 +33,7 @@ constexpr int kEpiWarps = 8;
 constexpr int kMaxSplit = 4;
 constexpr int kThreads = 32 * (2 + kEpiWarps);
 
-__host__ __device__ constexpr int stages_for(int bn) { return bn >= 256 ? 4 : (bn >= 128 ? 6 : 8); }
+__host__ __device__ constexpr int stages_for(int bn) { return bn >= 192 ? 4 : (bn >= 128 ? 6 : 8); }
 constexpr size_t smem_for(int bn) {
     return 1024 + static_cast<size_t>(stages_for(bn)) * (BM * BKB + bn * BKB) + kEpiWarps * 4096 + 256;
 }
@@ -116,7 +116,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     constexpr int kABytes = BM * BKB;
     constexpr int kBBytes = BN * BKB;
     constexpr int kStageBytes = kABytes + kBBytes;
-    constexpr uint32_t kTmemCols = 2 * BN;
+    constexpr uint32_t kTmemCols = BN == 192 ? 512 : 2 * BN;          // a power of two
     constexpr int LDS = BN + 4;                                        // floats per row of a share's sums
     static_assert(!SHARED || sizeof(float) * BM * LDS <= kStages * kStageBytes, "the sums take the stages' place");
     uint8_t* epi_stage = smem + kStages * kStageBytes;                 // 8 warps x 4 KB
@@ -328,7 +328,8 @@ cudaError_t launch_kernel(const CUtensorMap& ma, const CUtensorMap& mb, const Pa
 }
 template <int BN>
 cudaError_t launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t st) {
-    if (p.split > 1) return launch_kernel<BN, false, true>(ma, mb, p, st);
+    if constexpr (BN != 192)
+        if (p.split > 1) return launch_kernel<BN, false, true>(ma, mb, p, st);
     return p.c.residual ? launch_kernel<BN, true, false>(ma, mb, p, st) : launch_kernel<BN, false, false>(ma, mb, p, st);
 }
 
@@ -350,16 +351,17 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     // Tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
     // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to
     // measurements.  64 x 12288 x 4096: 64 tiles of 64 columns took 62 us, 32 of 128 in four shares 23; 512 x 6144 x 2048:
-    // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.
+    // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.  192 columns, whole tiles only, where 256 leave much of a last wave
+    // empty and 128 take one more (64 rows of the width-4096 model: 16 tokens 0.6 % shorter; 900-token prompts at width 2048: 0.7 %).
     const long long tm = (c.M + BM - 1) / BM, kb = (c.K + BKE - 1) / BKE;
     const int a_rows = c.M < 64 ? 64 : (c.M < BM ? static_cast<int>(c.M) : BM);
     int bn = 64, split = 1;
     double best = 0.0;
-    for (int b = 256; b >= 64; b /= 2) {
+    for (const int b : {256, 192, 128, 64}) {
         if (b > 64 && c.N <= b / 2) continue;
         const long long tiles = tm * ((c.N + b - 1) / b);
         for (int s = 1; s <= kMaxSplit; s *= 2) {
-            if (s > 1 && (kb < 4 * s || tiles * s > cluster_room<dense_tcgen05_kernel<256, false, true>>(s, kThreads, smem_for(256)))) break;
+            if (s > 1 && (b == 192 || kb < 4 * s || tiles * s > cluster_room<dense_tcgen05_kernel<256, false, true>>(s, kThreads, smem_for(256)))) break;
             const double blocks = static_cast<double>((tiles + kNumSm - 1) / kNumSm) * ((kb + s - 1) / s);
             const double us = blocks * (0.12 + 0.95e-3 * (a_rows + b)) + (s > 1 ? 1.7 + 3.9e-4 * a_rows * b / s : 0.0);
             if (best == 0.0 || us < best) { best = us; bn = b; split = s; }
@@ -372,6 +374,7 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     if (!make_map(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.x, c.M, c.K, BKE, BM, CU_TENSOR_MAP_SWIZZLE_128B, c.ldx))
         return cudaErrorUnknown;
     if (!make_map(&mb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.w, c.N, c.K, BKE, bn, CU_TENSOR_MAP_SWIZZLE_128B, c.ldw)) return cudaErrorUnknown;
+    if (bn == 192) return launch_bn<192>(ma, mb, p, st);
     return bn == 256 ? launch_bn<256>(ma, mb, p, st) : (bn == 128 ? launch_bn<128>(ma, mb, p, st) : launch_bn<64>(ma, mb, p, st));
 }
 

@@ -114,6 +114,27 @@ def test_dense_shares_of_k(cuda, stack_lib, m, k, n, ff):
     assert stack_lib.tbl_device_status(stream(torch)) == 0
 
 
+@pytest.mark.parametrize("m,k,n", [(64, 520, 148 * 192), (17, 264, 148 * 192 - 40), (130, 200, 74 * 192 - 7), (33, 1032, 149 * 192 + 64)])
+def test_dense_tiles_of_192_columns(cuda, stack_lib, m, k, n):
+    """A wave of them exactly, with a ragged end, and (the last) a few more than that; the residual in place, and the gated form."""
+    from reimagined_b200.stack import StackEngine
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, w, ff = torch.randn(m, k).bfloat16().cuda(), (torch.randn(n, k) * k ** -0.5).bfloat16(), n // 2
+    out = torch.randn(m, n, device="cuda")
+    want = out.double() + x.double() @ w.cuda().double().T
+    assert stack_lib.tbl_dense_forward(C.byref(b.view(w)), 1, TENSOR, x.data_ptr(), k, m, out.data_ptr(), out.data_ptr(), stream(torch)) == 0
+    assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-5
+    gate, up = w[:ff], w[ff:2 * ff]
+    h = torch.full((m, ff), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert stack_lib.tbl_gated_dense_forward(C.byref(b.view(StackEngine._paired(None, gate, up))), 1, TENSOR, x.data_ptr(), k, m, ff, h.data_ptr(),
+                                             stream(torch)) == 0
+    gw, uw = (x.double() @ v.cuda().double().T for v in (gate, up))
+    assert_close(f64(h), (torch.nn.functional.silu(gw) * uw).cpu().numpy(), 4e-3)
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 264, 148 * 16), (1, 5000, 148 * 16 + 1), (8, 512, 1200), (16, 520, 148 * 64), (9, 520, 148 * 64 + 9), (3, 264, 32000), (16, 2056, 37888),
                                    (1, 5000, 148 * 16 - 7), (8, 4104, 148 * 16 - 7), (9, 2056, 37889), (16, 2056, 37889)])
 def test_dense_rows_by_the_number_of_blocks(cuda, stack_lib, m, k, n):
