@@ -212,7 +212,10 @@ __global__ void __launch_bounds__(32 * kQuarters * MAPS) attention_stream_kernel
                         make_float2(o[j][q][2 * h], o[j][q][2 * h + 1]);
         }
     __syncthreads();
-    pdl_launch_dependents();
+    // With more than one block to an SM these leave no room on theirs, and up to 16 rows the output projection's blocks (dense_rows.cu) would crowd onto the SMs
+    // that have none: they come when these are done (16 sequences of the width-4096 Goguvik: a step 774 and 620 us).  More rows are the GEMM's, one block an SM,
+    // whom it helps to come early (64 sequences 653 and 637 us), as it helps where every SM has room (8 sequences of width 2048: 448 and 436).
+    if (gridDim.x * gridDim.y * gridDim.z <= kNumSm || gridDim.x / p.G * p.n_tok > 16) pdl_launch_dependents();
     // the quarters come together: sums of this split, a warp per row
     const size_t quarter_step = static_cast<size_t>(MAPS) * kRows * p.vp;
     const int rows = min(kRows, total - first);
