@@ -2,9 +2,9 @@
 // gemm_tcgen05.cu, with the same roles and the same operand geometry (a stage is 128 bytes of K per row, i.e. 64
 // bf16, in the 128-byte-swizzled K-major layout TMA writes; an MMA takes 32 bytes of K).
 //
-// One persistent CTA per SM (or, where the tiles would leave SMs idle, a cluster of CTAs per tile that share its K range and
-// finish it together), ten warps: TMA producer, MMA issuer (tcgen05.mma kind::f16, fp32 accumulators in TMEM,
-// two buffers of BN columns), eight epilogue warps.  128 x BN tiles; the two accumulators double-buffer tiles.  (256 x
+// One persistent CTA per SM -- two of them up to 64 rows -- (or, where the tiles would leave SMs idle, a cluster of CTAs per tile that share its K
+// range and finish it together), ten warps (six): TMA producer, MMA issuer (tcgen05.mma kind::f16, fp32 accumulators in TMEM,
+// two buffers of BN columns), eight (four) epilogue warps.  128 x BN tiles; the two accumulators double-buffer tiles.  (256 x
 // 256 tiles, which the int8 kernel uses for large problems, gain nothing here: these epilogues -- residual, gated pair --
 // are longer, and a tall tile cannot hide them.)
 // The epilogue adds the bias and either adds the fp32 residual and stores fp32, stores bf16, or -- for a gated
@@ -28,20 +28,24 @@ constexpr int BM = 128;             // activation rows per MMA
 constexpr int BKB = 128;            // bytes of K per stage
 constexpr int BKE = BKB / 2;        // the same in elements
 constexpr int kGroupM = 16;         // row tiles per group of the tile walk
-constexpr int kMaxStages = 8;
-constexpr int kEpiWarps = 8;
+constexpr int kMaxStages = 12;
 constexpr int kMaxSplit = 4;
-constexpr int kThreads = 32 * (2 + kEpiWarps);
+__host__ __device__ constexpr int threads_for(int ar) { return 32 * (2 + ar / 16); }
 
-__host__ __device__ constexpr int stages_for(int bn) { return bn >= 192 ? 4 : (bn >= 128 ? 6 : 8); }
-constexpr size_t smem_for(int bn) {
-    return 1024 + static_cast<size_t>(stages_for(bn)) * (BM * BKB + bn * BKB) + kEpiWarps * 4096 + 256;
+// ar: activation rows of a stage, 128, or 64 for no more than that (see the kernel).  With 64 two CTAs share an SM.
+__host__ __device__ constexpr int epi_warps(int ar) { return ar / 16; }
+constexpr size_t other_smem(int ar) { return (ar == BM ? 1024 : 0) + epi_warps(ar) * 4096 + 256; }
+// deep: where an SM has one CTA anyway, stages to fill it
+__host__ __device__ constexpr int stages_for(int bn, int ar, bool deep) {
+    return ar == BM ? (bn >= 192 ? 4 : (bn >= 128 ? 6 : 8)) : (bn >= 128 ? 4 : 6) * (deep ? 2 : 1);
 }
+constexpr size_t smem_for(int bn, int ar, bool deep) { return other_smem(ar) + static_cast<size_t>(stages_for(bn, ar, deep)) * (ar + bn) * BKB; }
 
 struct Params {
     DenseCall c;
     int tiles_m, tiles_n;
     int split;              // shares of K = CTAs of a cluster (SHARED kernel)
+    int deep;               // 64 rows: all of an SM's shared memory for one CTA
     int vec;                // outputs (and residual) take 4-column vector accesses
     int* status;
 };
@@ -107,26 +111,38 @@ __device__ __forceinline__ void store_block(const Params& p, const uint8_t* stag
 }
 
 // SHARED: a CTA takes one share of the K range of one tile, the CTAs of a cluster finish the tile together.
-template <int BN, bool RES, bool SHARED>
-__global__ void __launch_bounds__(kThreads, 1)
+// AR: activation rows of a stage, 128, or 64 for no more rows than that: the MMA still takes 128, the upper half of them from the weights behind (of the
+// same stage), and nobody reads those sums.
+// With so few rows a layer is the stream of its weights, and what held that up was the chain of a K block in the two issuing warps (0.33 us a block however
+// narrow the tile; one elected lane, places counted instead of divided for, descriptors by addition: 0.18) and that nothing streams while a block of one CTA
+// to an SM starts up or stores.  So two CTAs share an SM, each with half of its memory, except where there are no more CTAs than SMs and K is long: then one
+// has twice the stages.  us before | after at 64 rows, cold weights: 24576 gated x 4096 53.2 | 43.1, 32000 x 4096 53.9 | 47.3, 8192 x 4096 18.9 | 17.4,
+// 4096 x 12288 24.6 | 23.2, 2048 x 6144 13.2 | 10.8, 10304 x 2048 15.4 | 12.1.  A step of 64 sequences of the width-4096 Guselix 803 | 762, of 32 of the
+// width-2048 Goguvik 577 | 523, of 24 of the width-2048 Guselix 746 | 642.
+template <int BN, int AR, bool RES, bool SHARED>
+__global__ void __launch_bounds__(threads_for(AR), AR == BM ? 1 : 2)
 dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Params p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int kStages = stages_for(BN);
-    constexpr int kABytes = BM * BKB;
+    // (nothing else is in shared memory, which starts on a 1024-byte boundary as declared; with two CTAs there is no room to round up)
+    uint8_t* smem = AR == BM ? reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023)) : smem_raw;
+    constexpr int kThreads = threads_for(AR), kEpiWarps = epi_warps(AR);
+    const int kStages = AR == BM ? stages_for(BN, AR, false) : stages_for(BN, AR, p.deep);
+    constexpr int kLoadWarp = AR == BM ? 0 : 2, kMmaWarp = kLoadWarp + 1;   // the others are epilogue warps, which reach the TMEM lanes of their number mod 4
+    constexpr int kABytes = AR * BKB;
     constexpr int kBBytes = BN * BKB;
     constexpr int kStageBytes = kABytes + kBBytes;
     constexpr uint32_t kTmemCols = BN == 192 ? 512 : 2 * BN;          // a power of two
     constexpr int LDS = BN + 4;                                        // floats per row of a share's sums
-    static_assert(!SHARED || sizeof(float) * BM * LDS <= kStages * kStageBytes, "the sums take the stages' place");
-    uint8_t* epi_stage = smem + kStages * kStageBytes;                 // 8 warps x 4 KB
+    static_assert(AR + BN >= BM, "the rows an MMA takes lie within the stage");
+    static_assert(!SHARED || sizeof(float) * AR * LDS <= stages_for(BN, AR, false) * kStageBytes, "the sums take the stages' place");
+    uint8_t* epi_stage = smem + kStages * kStageBytes;                 // 4 KB a warp
     uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + kEpiWarps * 4096);
     uint64_t* empty = full + kMaxStages;
     uint64_t* tmem_full = empty + kMaxStages;
     uint64_t* tmem_empty = tmem_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int all_blocks = (p.c.K + BKE - 1) / BKE, per = SHARED ? (all_blocks + p.split - 1) / p.split : all_blocks;
     const int share = SHARED ? blockIdx.x % p.split : 0, first = SHARED ? blockIdx.x / p.split : blockIdx.x;
     const int stride = SHARED ? p.tiles_m * p.tiles_n : gridDim.x;     // SHARED: this tile only
@@ -138,7 +154,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         fence_mbar_init();
         fence_proxy_async();
     }
-    if (warp == 1) {
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -148,43 +164,54 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
+    // Up to 64 rows every tile starts at another block of K: otherwise all of them would ask for the same few lines of the activations at the same time
+    // (64 x 24576 x 4096 45.3 and 43.1 us, 64 x 32000 x 4096 49.2 and 47.3; a step of 64 sequences of the width-4096 Goguvik 601 and 583).
+    auto k_block = [&](int kb, int tn) {
+        if (AR == BM) return kb0 + kb;
+        const int at = kb + tn * 7 % kblocks;
+        return kb0 + (at < kblocks ? at : at - kblocks);
+    };
     // the weights of the first stages do not depend on the kernel before this one, unless the call says so
     int early = 0;
-    if (warp == 0) {
+    if (warp == kLoadWarp) {
         int row0, tn;
         if (!p.c.w_computed && decode_tile(p, first, row0, tn)) early = min(kStages, kblocks);
-        if (lane == 0)
+        if (elect_one())
             for (int s = 0; s < early; ++s) {
                 mbar_arrive_expect_tx(&full[s], kStageBytes);
-                tma_load_2d(smem + s * kStageBytes + kABytes, &map_b, (kb0 + s) * BKE, tn * BN, &full[s]);
+                tma_load_2d(smem + s * kStageBytes + kABytes, &map_b, k_block(s, tn) * BKE, tn * BN, &full[s]);
             }
     }
     pdl_wait();
 
-    if (warp == 0) {
+    if (warp == kLoadWarp) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int it = 0, row0, tn;
+        if (elect_one()) {
+            int s = 0, row0, tn;
+            uint32_t round = 0;                                // full rounds of the ring so far
             bool alive = true;
             for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride) {
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % kStages;
-                    if (it >= kStages) {
-                        alive = mbar_wait_bounded(&empty[s], ((it / kStages) - 1) & 1, p.status);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (round) {
+                        alive = mbar_wait_bounded(&empty[s], (round - 1) & 1, p.status);
                         if (!alive) break;
                     }
                     uint8_t* a_dst = smem + s * kStageBytes;
-                    if (it >= early) mbar_arrive_expect_tx(&full[s], kStageBytes);
-                    tma_load_2d(a_dst, &map_a, (kb0 + kb) * BKE, row0, &full[s]);
-                    if (it >= early) tma_load_2d(a_dst + kABytes, &map_b, (kb0 + kb) * BKE, tn * BN, &full[s]);
+                    const bool whole = round || s >= early;
+                    if (whole) mbar_arrive_expect_tx(&full[s], kStageBytes);
+                    tma_load_2d(a_dst, &map_a, k_block(kb, tn) * BKE, row0, &full[s]);
+                    if (whole) tma_load_2d(a_dst + kABytes, &map_b, k_block(kb, tn) * BKE, tn * BN, &full[s]);
+                    if (++s == kStages) { s = 0; ++round; }
                 }
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == kMmaWarp) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = idesc_bf16(BN);
-            int it = 0, local = 0, row0, tn;
+            const uint64_t a_desc = smem_desc_sw128(smem_u32(smem)), b_desc = smem_desc_sw128(smem_u32(smem) + kABytes);
+            int s = 0, local = 0, row0, tn;
+            uint32_t phase = 0;
             bool alive = true;
             for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride, ++local) {
                 const int buf = local & 1;
@@ -194,24 +221,22 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % kStages;
-                    alive = mbar_wait_bounded(&full[s], (it / kStages) & 1, p.status);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    alive = mbar_wait_bounded(&full[s], phase, p.status);
                     if (!alive) break;
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
-                    const uint32_t b_addr = a_addr + kABytes;
+                    const uint32_t at = static_cast<uint32_t>(s) * (kStageBytes >> 4);     // descriptors count 16 bytes
 #pragma unroll
-                    for (int kk = 0; kk < BKB / 32; ++kk)
-                        umma_f16(d_tmem, smem_desc_sw128(a_addr + kk * 32), smem_desc_sw128(b_addr + kk * 32), idesc, (kb | kk) != 0 ? 1u : 0u);
+                    for (int kk = 0; kk < BKB / 32; ++kk) umma_f16(d_tmem, a_desc + at + 2 * kk, b_desc + at + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
                     umma_commit(&empty[s]);
+                    if (++s == kStages) { s = 0; phase ^= 1; }
                 }
                 if (alive) umma_commit(&tmem_full[buf]);
             }
         }
     } else if (SHARED) {
         // ---------------- sums of this share into the place of the stages (all of which the MMAs have read) ----------------
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int quarter = warp & 3, half = AR == BM ? (warp - 2) >> 2 : warp >> 2;
         float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * LDS + half * (BN / 2);
         bool alive = mbar_wait_bounded(&tmem_full[0], 0, p.status);     // (no share is empty: K has four blocks for each)
         alive = __all_sync(0xffffffffu, alive);
@@ -228,8 +253,8 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else {
         // ---------------- epilogue warps ----------------
         const int quarter = warp & 3;          // TMEM lanes 32*quarter .. +31 are this warp's
-        const int half = (warp - 2) >> 2;      // which of the two warps of the quarter
-        uint8_t* stage = epi_stage + (warp - 2) * 4096;
+        const int half = AR == BM ? (warp - 2) >> 2 : warp >> 2;      // which of the two warps of the quarter
+        uint8_t* stage = epi_stage + (AR == BM ? warp - 2 : 2 * half + quarter) * 4096;
         const bool pair = p.c.pair_cols > 0;
         const Activation act = activation_of(p.c.act);
         int local = 0, tile_row0, tn;
@@ -302,35 +327,45 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         decode_tile(p, first, row0, tn);
         __syncwarp();
         cluster_sync_all();
-        finish_shares<BN, LDS, kThreads>(p.c, smem_u32(smem), p.split, share, tn, row0, BM, p.vec, [](int, int, float v) { return v; });
+        finish_shares<BN, LDS, kThreads>(p.c, smem_u32(smem), p.split, share, tn, row0, AR, p.vec, [](int, int, float v) { return v; });
         cluster_sync_all();                                // nobody leaves while a neighbour may still read its sums
     }
 
     // common exit: all roles meet, then the allocating warp releases TMEM
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == kMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
 }
 
-template <int BN, bool RES, bool SHARED>
+template <int BN, int AR, bool RES, bool SHARED>
 cudaError_t launch_kernel(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t st) {
     static bool done[64] = {};
-    constexpr size_t smem = smem_for(BN);
-    static_assert(smem <= 227 * 1024, "shared memory of a CTA");
-    const cudaError_t e = allow_smem(dense_tcgen05_kernel<BN, RES, SHARED>, smem, done);
+    constexpr size_t most = smem_for(BN, AR, true);
+    static_assert(most <= 227 * 1024 && (AR == BM || smem_for(BN, AR, false) <= 113 * 1024), "shared memory of a CTA");
+    const size_t smem = smem_for(BN, AR, p.deep);
+    const cudaError_t e = allow_smem(dense_tcgen05_kernel<BN, AR, RES, SHARED>, most, done);
     if (e != cudaSuccess) return e;
     const int tiles = p.tiles_m * p.tiles_n;
-    if (SHARED) return launch_dependent_cluster(dense_tcgen05_kernel<BN, RES, SHARED>, dim3(tiles * p.split), p.split, dim3(kThreads), smem, st, ma, mb, p);
-    return launch_dependent(dense_tcgen05_kernel<BN, RES, SHARED>, dim3(tiles < kNumSm ? tiles : kNumSm), dim3(kThreads), smem, st, ma, mb, p);
+    constexpr int kThreads = threads_for(AR), room = AR == BM ? kNumSm : 2 * kNumSm;
+    if (SHARED) return launch_dependent_cluster(dense_tcgen05_kernel<BN, AR, RES, SHARED>, dim3(tiles * p.split), p.split, dim3(kThreads), smem, st, ma, mb, p);
+    return launch_dependent(dense_tcgen05_kernel<BN, AR, RES, SHARED>, dim3(tiles < room ? tiles : room), dim3(kThreads), smem, st, ma, mb, p);
 }
-template <int BN>
+template <int BN, int AR>
 cudaError_t launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, cudaStream_t st) {
     if constexpr (BN != 192)
-        if (p.split > 1) return launch_kernel<BN, false, true>(ma, mb, p, st);
-    return p.c.residual ? launch_kernel<BN, true, false>(ma, mb, p, st) : launch_kernel<BN, false, false>(ma, mb, p, st);
+        if (p.split > 1) return launch_kernel<BN, AR, false, true>(ma, mb, p, st);
+    return p.c.residual ? launch_kernel<BN, AR, true, false>(ma, mb, p, st) : launch_kernel<BN, AR, false, false>(ma, mb, p, st);
+}
+template <int AR>
+cudaError_t launch_ar(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, int bn, cudaStream_t st) {
+    if constexpr (AR == BM) {
+        if (bn == 256) return launch_bn<256, AR>(ma, mb, p, st);
+        if (bn == 192) return launch_bn<192, AR>(ma, mb, p, st);
+    }
+    return bn == 128 ? launch_bn<128, AR>(ma, mb, p, st) : launch_bn<64, AR>(ma, mb, p, st);
 }
 
 }  // namespace
@@ -348,34 +383,56 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     const int cols = c.pair_cols ? c.pair_cols : c.N;
     p.vec = (cols % 4 == 0) && (c.ldo % 4 == 0) && (reinterpret_cast<uintptr_t>(c.out_f32) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(c.out_b16) & 7) == 0 && (reinterpret_cast<uintptr_t>(c.residual) & 15) == 0;
-    // Tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
-    // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to
-    // measurements.  64 x 12288 x 4096: 64 tiles of 64 columns took 62 us, 32 of 128 in four shares 23; 512 x 6144 x 2048:
-    // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.  192 columns, whole tiles only, where 256 leave much of a last wave
-    // empty and 128 take one more (64 rows of the width-4096 model: 16 tokens 0.6 % shorter; 900-token prompts at width 2048: 0.7 %).
     const long long tm = (c.M + BM - 1) / BM, kb = (c.K + BKE - 1) / BKE;
     const int a_rows = c.M < 64 ? 64 : (c.M < BM ? static_cast<int>(c.M) : BM);
     int bn = 64, split = 1;
     double best = 0.0;
-    for (const int b : {256, 192, 128, 64}) {
-        if (b > 64 && c.N <= b / 2) continue;
-        const long long tiles = tm * ((c.N + b - 1) / b);
-        for (int s = 1; s <= kMaxSplit; s *= 2) {
-            if (s > 1 && (b == 192 || kb < 4 * s || tiles * s > cluster_room<dense_tcgen05_kernel<256, false, true>>(s, kThreads, smem_for(256)))) break;
-            const double blocks = static_cast<double>((tiles + kNumSm - 1) / kNumSm) * ((kb + s - 1) / s);
-            const double us = blocks * (0.12 + 0.95e-3 * (a_rows + b)) + (s > 1 ? 1.7 + 3.9e-4 * a_rows * b / s : 0.0);
-            if (best == 0.0 || us < best) { best = us; bn = b; split = s; }
+    if (c.M <= 64) {
+        // The chain of a CTA's K blocks (0.17 us and more each) against the weights' bytes at 6 TB/s, both felt where they are alike; plus storing the
+        // tile or exchanging the sums of shares.  us, fitted to 23 shapes at 64 and 24 rows: within a tenth of the best choice on 19 of them.  Beyond two CTAs an SM the last
+        // round counts whole.
+        const double mem = 2.0 * c.N * c.K / 6.0e6;
+        for (const int b : {128, 64}) {
+            if (b > 64 && c.N <= b / 2) continue;
+            const long long tiles = (c.N + b - 1) / b;
+            for (int s = 1; s <= kMaxSplit; s *= 2) {
+                const long long n = tiles * s;
+                if (s > 1 && (kb < 4 * s || n > cluster_room<dense_tcgen05_kernel<128, 64, false, true>>(s, threads_for(64), smem_for(128, 64, false)))) break;
+                // (up to 16 blocks of K the memory is better left to the kernel that comes next: 24 sequences at width 1024 397 and 378 us a step)
+                const bool deep = n <= (s > 1 ? 128 : kNumSm) && (kb + s - 1) / s > 16;
+                const long long waves = (n + 2 * kNumSm - 1) / (2 * kNumSm);
+                const double chain = static_cast<double>(waves * ((kb + s - 1) / s)) * (deep ? (b == 128 ? 0.18 : 0.17) : (b == 128 ? 0.29 : 0.2));
+                const double m = waves > 1 ? mem * (2.0 * kNumSm * waves) / n : mem;
+                const double us = sqrt(chain * chain + m * m) + (s > 1 ? 1.2 + 0.025 * b / s : 0.02 * b);
+                if (best == 0.0 || us < best) { best = us; bn = b; split = s; p.deep = deep; }
+            }
+        }
+    } else {
+        // More than 64 rows: tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
+        // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to
+        // measurements.  64 x 12288 x 4096: 64 tiles of 64 columns took 62 us, 32 of 128 in four shares 23; 512 x 6144 x 2048:
+        // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.  192 columns, whole tiles only, where 256 leave much of a last wave
+        // empty and 128 take one more (64 rows of the width-4096 model: 16 tokens 0.6 % shorter; 900-token prompts at width 2048: 0.7 %).
+        for (const int b : {256, 192, 128, 64}) {
+            if (b > 64 && c.N <= b / 2) continue;
+            const long long tiles = tm * ((c.N + b - 1) / b);
+            for (int s = 1; s <= kMaxSplit; s *= 2) {
+                if (s > 1 && (b == 192 || kb < 4 * s || tiles * s > cluster_room<dense_tcgen05_kernel<256, BM, false, true>>(s, threads_for(BM), smem_for(256, BM, true)))) break;
+                const double blocks = static_cast<double>((tiles + kNumSm - 1) / kNumSm) * ((kb + s - 1) / s);
+                const double us = blocks * (0.12 + 0.95e-3 * (a_rows + b)) + (s > 1 ? 1.7 + 3.9e-4 * a_rows * b / s : 0.0);
+                if (best == 0.0 || us < best) { best = us; bn = b; split = s; }
+            }
         }
     }
     p.split = split;
+    const int ar = c.M <= 64 ? 64 : BM;
     p.tiles_m = static_cast<int>(tm);
     p.tiles_n = (c.N + bn - 1) / bn;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.x, c.M, c.K, BKE, BM, CU_TENSOR_MAP_SWIZZLE_128B, c.ldx))
+    if (!make_map(&ma, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.x, c.M, c.K, BKE, ar, CU_TENSOR_MAP_SWIZZLE_128B, c.ldx))
         return cudaErrorUnknown;
     if (!make_map(&mb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.w, c.N, c.K, BKE, bn, CU_TENSOR_MAP_SWIZZLE_128B, c.ldw)) return cudaErrorUnknown;
-    if (bn == 192) return launch_bn<192>(ma, mb, p, st);
-    return bn == 256 ? launch_bn<256>(ma, mb, p, st) : (bn == 128 ? launch_bn<128>(ma, mb, p, st) : launch_bn<64>(ma, mb, p, st));
+    return ar == 64 ? launch_ar<64>(ma, mb, p, bn, st) : launch_ar<BM>(ma, mb, p, bn, st);
 }
 
 }  // namespace stack
