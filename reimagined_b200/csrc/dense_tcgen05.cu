@@ -163,7 +163,7 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_launch_dependents();
+    if (AR == BM) pdl_launch_dependents();
     // Up to 64 rows every tile starts at another block of K: otherwise all of them would ask for the same few lines of the activations at the same time
     // (64 x 24576 x 4096 45.3 and 43.1 us, 64 x 32000 x 4096 49.2 and 47.3; a step of 64 sequences of the width-4096 Goguvik 601 and 583).
     auto k_block = [&](int kb, int tn) {
@@ -183,6 +183,10 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
     }
     pdl_wait();
+    // Up to 64 rows not before the wait (24 sequences at width 2048 646 and 640 us a step: dense_rows.cu says why), and up to 16, where the layers around are the
+    // row-streaming kernel's, whose blocks crowd onto the SMs without one of these, not at all (16 sequences of the width-4096 Guselix 866 and 714,
+    // of the width-2048 one 718 and 606).
+    if (AR != BM && p.c.M > 16) pdl_launch_dependents();
 
     if (warp == kLoadWarp) {
         // ---------------- TMA producer ----------------
