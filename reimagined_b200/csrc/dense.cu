@@ -243,18 +243,23 @@ bool gemv_supported(const DenseCall& c) {
     return c.M <= kGemvMaxRows && sizeof(float) * c.M * c.K <= kGemvMaxSmem && (c.K % 4 == 0 || c.M == 1);
 }
 
-// Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 16 rows, except that more than eight rows of a
-// long K are better shared out (16 x 12288 x 4096: 32 and 23 us; 8 x 6144 x 2048: 9 and 12).  Up to 32 rows it does where
-// four or eight warps share K (32 x 512 x 2048: 0.74 of the GEMM's time, 32 x 2048 x 2048 0.80, 32 x 4096 x 2048 0.97; but 1.3
-// .. 2.6 at K of 256 and less, 1.2 at 8192) and the matrix is no more than a wave of blocks (17 x 1024 x 4096 0.96, 17 x 2048 x
-// 4096 1.21, 17 x 512 x 8192 1.15); up to 48 rows with eight warps of the shortest share (48 x 1024 x 2048 0.81, 48 x 768 x
-// 2048 1.31, 48 x 1536 x 1024 1.29).  Beyond that never: 512 x 64 x 2048 takes it 14 us and the GEMM 3.2.
+// Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 8 rows.  Up to 16 it does for gated layers (us, rows and GEMM: 16 x 12288 x 2048
+// 12.4 and 18 .. 23, 24576 x 4096 41 and 43) and except where, with some K, the matrix is very tall (16 x 16384 x 2048 25.8 and 20.1, 32000 x 4096 86 and 46;
+// but 10304 x 2048 13.6 and 17.0) or its blocks are a little more than a wave of three to an SM (N of 7105 .. 8288: 8192 x 4096 24.6 and 15.6, 8192 x 2048 14.2
+// and 11.6; but 8192 x 1024 8.8 and 8.7), or where K is long beside N, which the GEMM shares out (4096 x 12288 32 and 22).  A step with the first two: 16
+// sequences of the width-4096 Guselix 714 and 627, of width 3072 500 and 459, 10 of the width-4096 Goguvik 577 and 535.  Lines that only the layers by
+// themselves bear out are not drawn: 4096 x 4096 takes 13.0 and 11.4, steps with it by the GEMM are up to a fourth longer, and 32000 x 1024 26 and 17, but
+// steps 2 % longer.
+// Up to 32 rows it does where eight warps share a short K and the matrix is no more than a wave of blocks (17 x 2048 x 512 4.1 and 4.8, 32 x 2048 x 1024 4.6
+// and 5.5, 17 x 2048 x 2048 6.3 and 6.4; but 17 x 2048 x 3072 8.1 and 7.4, 17 x 4096 x 1024 7.6 and 6.5).  Beyond that never (48 x 2048 x 1024 5.8 and 5.7,
+// 512 x 64 x 2048 14 and 3.2).
 bool rows_pay(const DenseCall& c) {
-    const long long size = static_cast<long long>(c.N) * c.K;
     if (c.batch > 0 || c.M <= 8) return true;
-    if (c.M <= 16) return c.K < 2LL * c.N || size < (12 << 20);
-    if (c.M <= 32) return c.K >= 512 && c.K <= 4096 && (c.N <= 2048 || (c.N <= 4096 && c.K <= 1024));
-    return c.M <= 48 && c.K >= 1024 && c.K < 1536 && c.N <= 2048;
+    if (c.M <= 16) {
+        if (c.K >= 2048 && !c.pair_cols && (c.N > 14208 || (c.N > 7104 && c.N <= 8288))) return false;
+        return c.K < 2LL * c.N || static_cast<long long>(c.N) * c.K < (12 << 20);
+    }
+    return c.M <= 32 && c.K >= 512 && c.K <= 2048 && (c.N <= 2048 || (c.N <= 4096 && c.K < 1024));
 }
 
 }  // namespace

@@ -178,6 +178,25 @@ def test_dense_of_many_rows_is_the_gemm(cuda, stack_lib, m, k, n):
     assert torch.equal(outs[0], outs[1]) and not torch.equal(outs[0], outs[2])           # (the two add up in different orders)
 
 
+@pytest.mark.parametrize("m,k,n,route", [(8, 2048, 16384, ROWS), (9, 2048, 14208, ROWS), (9, 2048, 14209, TENSOR), (9, 2040, 14209, ROWS), (16, 2048, 7104, ROWS),
+                                         (16, 2048, 7105, TENSOR), (9, 2048, 8288, TENSOR), (9, 2048, 8289, ROWS), (16, 2040, 8000, ROWS), (9, 6136, 2048, ROWS),
+                                         (9, 6144, 2048, TENSOR), (17, 1016, 4096, ROWS), (17, 1024, 2049, TENSOR), (32, 2048, 2048, ROWS), (32, 2056, 64, TENSOR),
+                                         (33, 1024, 512, TENSOR)])
+def test_dense_route_of_few_rows(cuda, stack_lib, m, k, n, route):
+    """Either side of every line of the rule: the route it names, bit for bit, and both within rounding of 64 bits."""
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, w = torch.randn(m, k).bfloat16().cuda(), torch.randn(n, k).bfloat16()
+    view, outs = b.view(w), {}
+    want = x.double() @ w.cuda().double().T
+    for r in (0, TENSOR, ROWS):
+        outs[r] = torch.full((m, n), float("nan"), device="cuda")
+        assert stack_lib.tbl_dense_forward(C.byref(view), 1, r, x.data_ptr(), k, m, None, outs[r].data_ptr(), stream(torch)) == 0
+        assert float((outs[r].double() - want).abs().max() / want.abs().max()) < 1e-5
+    assert torch.equal(outs[0], outs[route]) and not torch.equal(outs[TENSOR], outs[ROWS])
+
+
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
 @pytest.mark.parametrize("m,k,ff", [(9, 512, 70), (1, 64, 32), (3, 40, 37), (4, 128, 200), (1, 1024, 3000), (150, 72, 100), (260, 136, 333)])
 def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
@@ -746,6 +765,25 @@ def test_stream_norm(cuda, stack_lib, precision, rows, width, streams):
             assert_close(f64(h), want, tol, "h")
             for got, a in zip(f64(x), new if store else xs):
                 assert_close(got, a, 3e-6 if store else 0, "streams")
+
+
+@pytest.mark.parametrize("m,k,n,route", [(8, 2048, 16384, ROWS), (9, 2048, 14208, ROWS), (9, 2048, 14209, TENSOR), (9, 2040, 14209, ROWS), (16, 2048, 7104, ROWS),
+                                         (16, 2048, 7105, TENSOR), (9, 2048, 8288, TENSOR), (9, 2048, 8289, ROWS), (16, 2040, 8000, ROWS), (9, 6136, 2048, ROWS),
+                                         (9, 6144, 2048, TENSOR), (17, 1016, 4096, ROWS), (17, 1024, 2049, TENSOR), (32, 2048, 2048, ROWS), (32, 2056, 64, TENSOR),
+                                         (33, 1024, 512, TENSOR)])
+def test_dense_route_of_few_rows(cuda, stack_lib, m, k, n, route):
+    """Either side of every line of the rule: the route it names, bit for bit, and both within rounding of 64 bits."""
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, w = torch.randn(m, k).bfloat16().cuda(), torch.randn(n, k).bfloat16()
+    view, outs = b.view(w), {}
+    want = x.double() @ w.cuda().double().T
+    for r in (0, TENSOR, ROWS):
+        outs[r] = torch.full((m, n), float("nan"), device="cuda")
+        assert stack_lib.tbl_dense_forward(C.byref(view), 1, r, x.data_ptr(), k, m, None, outs[r].data_ptr(), stream(torch)) == 0
+        assert float((outs[r].double() - want).abs().max() / want.abs().max()) < 1e-5
+    assert torch.equal(outs[0], outs[route]) and not torch.equal(outs[TENSOR], outs[ROWS])
 
 
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
