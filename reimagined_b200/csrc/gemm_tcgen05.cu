@@ -134,7 +134,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* tmem_empty = tmem_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int kblocks = (p.K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
@@ -155,17 +155,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int it = 0;
+        if (elect_one()) {
+            int s = 0;
+            uint32_t round = 0;                                // full rounds of the ring so far
             bool alive = true;
             int g, row0, rows, tn;
             for (int tile = blockIdx.x; alive && decode_tile<GROUPED, MT>(p, gt, tile, g, row0, rows, tn); tile += gridDim.x) {
                 const CUtensorMap* bmap = &map_b;
                 if constexpr (GROUPED) bmap = &gt.b[g];
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % kStages;
-                    if (it >= kStages) {
-                        alive = mbar_wait_bounded(&empty[s], ((it / kStages) - 1) & 1, p.status);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (round) {
+                        alive = mbar_wait_bounded(&empty[s], (round - 1) & 1, p.status);
                         if (!alive) break;
                     }
                     uint8_t* a_dst = smem + s * kStageBytes;
@@ -176,16 +176,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tma_load_2d(a_dst, &map_a, kb * BK, row0, &full[s]);
                     if constexpr (MT == 2) tma_load_2d(a_dst + BM * BK, &map_a, kb * BK, row0 + BM, &full[s]);
                     tma_load_2d(b_dst, bmap, kb * BK, tn * BN, &full[s]);
+                    if (++s == kStages) { s = 0; ++round; }
                 }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             // kind::i8 instruction descriptor: D = s32, A = B = signed 8-bit, both K-major, N = BN, M = 128
             const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
                                    (static_cast<uint32_t>(BM >> 4) << 24);
-            int it = 0, local = 0;
+            // An elected thread, places counted and descriptors by addition: a K block cost the issuing thread about 0.3 us otherwise, which narrow tiles waited for.
+            const uint64_t a_desc = smem_desc_sw128(smem_u32(smem)), b_desc = smem_desc_sw128(smem_u32(smem) + kABytes);
+            int s = 0, local = 0;
+            uint32_t phase = 0;
             bool alive = true;
             int g, row0, rows, tn;
             for (int tile = blockIdx.x; alive && decode_tile<GROUPED, MT>(p, gt, tile, g, row0, rows, tn);
@@ -202,13 +206,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 // drains half 0 first, so this tile's first MMAs run while half 1 is still being stored)
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (MT == 1 ? buf * BN : 0);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % kStages;
-                    alive = mbar_wait_bounded(&full[s], (it / kStages) & 1, p.status);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    alive = mbar_wait_bounded(&full[s], phase, p.status);
                     if (!alive) break;
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
-                    const uint32_t b_addr = a_addr + kABytes;
+                    const uint32_t at = static_cast<uint32_t>(s) * (kStageBytes >> 4);     // descriptors count 16 bytes
 #pragma unroll
                     for (int h = 0; h < MT; ++h) {
                         if constexpr (MT == 2) {
@@ -220,12 +222,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         }
 #pragma unroll
                         for (int kk = 0; kk < BK / 32; ++kk) {
-                            umma_i8(d_tmem + h * BN, smem_desc_sw128(a_addr + h * (BM * BK) + kk * 32),
-                                    smem_desc_sw128(b_addr + kk * 32), idesc, (kb | kk) != 0 ? 1u : 0u);
+                            umma_i8(d_tmem + h * BN, a_desc + at + (h * (BM * BK) >> 4) + 2 * kk, b_desc + at + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
                         }
                     }
                     if (!alive) break;
                     umma_commit(&empty[s]);   // stage reusable once these MMAs have read it
+                    if (++s == kStages) { s = 0; phase ^= 1; }
                 }
                 if (alive) {
                     if constexpr (MT == 1) {
