@@ -41,7 +41,7 @@ constexpr int kMaxParts = 64;        // parts of a row's sum of squares
 constexpr int kMaxBlocks = 32;       // blocks of a launch (kernel parameters)
 constexpr int kTaps = 3;             // tokens before this one that the convolution sees
 constexpr int kJobs = 8;             // projections of a pass
-
+constexpr int kStripParts = 8;       // parts of a row's sum in the order kSumStrips
 
 struct Linear {
     const uint8_t* strips;
@@ -325,6 +325,8 @@ enum SumOrder {
     kSumClusters,    // mamba_mix_cluster_kernel: eight CTAs, `share` numbers each, one a thread
 };
 struct Sums { int order, share, row0; };      // row0: of the batch, the cluster's first
+// The most of that kernel's warps (32 threads of 16 numbers) that a row of K numbers lies in
+__host__ __device__ __forceinline__ int sum_strips_parts(int K) { return (K >> 9) + 2; }
 
 // The sums over the lanes of eight numbers a lane, each added up like a butterfly (lanes 16, 8, 4, 2, 1 apart), in nine exchanges: at each of the first
 // three steps a lane keeps half of its numbers and sends the others.  Lane l has number l / 4 in the end.
@@ -345,10 +347,11 @@ __device__ __forceinline__ void sum_parts(const Sums& o, const float* src, int K
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (o.order == kSumStrips) {
         // its warps in order: of a row that goes on at the first warp, the parts there come first
-        const int n = (K >> 9) + 2;
+        static_assert(kStripParts == 8, "sum_total() adds eight");
+        const int n = sum_strips_parts(K);
 #pragma unroll 1
-        for (int i = warp; i < R * 8; i += T / 32) {
-            const int r = ONE ? 0 : i >> 3, p = i & 7;
+        for (int i = warp; i < R * kStripParts; i += T / 32) {
+            const int r = ONE ? 0 : i / kStripParts, p = i % kStripParts;
             const int g0 = (o.row0 + r) * (K >> 4), w0 = g0 >> 5, g = (w0 + p) * 32 + lane - g0, wrap = 16 - (w0 & 15);
             float ss = 0.0f;
             if (p < n) {
@@ -1391,6 +1394,8 @@ bool decode_cluster_shape(const tbl_decode_model& m, int batch, int capacity, Cl
     Dims d;
     int score_len;
     if (!common_dims(m, capacity, &d, &score_len)) return false;
+    // the parts that gemv_strip_kernel takes a row's sum of squares in: more than sum_parts() has places for
+    if (batch <= gemv_strip_fused_rows(d.D) && sum_strips_parts(d.D) > kStripParts) return false;
     for (int ctas = 16; ctas >= 8; ctas >>= 1) {
         const int most = clusters_at_once(ctas);
         if (most <= 0) continue;

@@ -51,6 +51,34 @@ def test_blocks_in_clusters_match_separate_launches(cuda, tbl, change, rows):
     assert clusters.capture() <= 6 < general.capture()
 
 
+class Inner(int):
+    """Stands where a configuration has the factor between model width and channels: any width gives this many."""
+
+    def __mul__(self, width):
+        return int(self)
+
+
+@pytest.mark.parametrize("width,rows,in_clusters", [
+    (3328, 1, True), (3328, 4, True),                            # as many parts of a row's sum of squares as the kernel adds: 8
+    (3584, 1, False), (3584, 4, False), (4096, 2, False), (4352, 1, False), (4608, 3, False),      # more: separate launches
+    (3584, 5, True),                                             # so many rows that the sum is taken in the other order, of any width
+])
+def test_residual_stream_wider_than_the_channels(cuda, tbl, width, rows, in_clusters):
+    """A row's sum of squares is added up in the parts that the separate launches take it in, of which a wide row has more than the kernel has places for."""
+    import gpu_helpers as H
+    cfg = dict(BASE, d_model=width, mamba_expand=Inner(1024), num_layers=3, attention_period=9)
+    _, clusters, general = engines(cfg, rows, 8)
+    rng = np.random.default_rng(width)
+    for t in range(3):
+        ids = rng.integers(0, cfg["vocab_size"], rows).tolist()
+        got, hidden = clusters.step(ids, trace=True)
+        want, hidden_want = general.step(ids, trace=True)
+        assert cuda.equal(hidden, hidden_want), f"token {t}: first block off {(hidden != hidden_want).flatten(1).any(dim=1).nonzero()[0]}"
+        assert cuda.equal(got, want), f"token {t}"
+    assert H.device_status() == 0
+    assert (clusters.capture() <= 5) == in_clusters
+
+
 def test_long_context_matches_separate_launches_to_rounding(cuda, tbl):
     """300 cached tokens: keys read by four lanes a token.  Scores in another order of sums, 1e-6 of their size, now and then move an 8-bit code by a
     step: 1 / 127 of the row's largest value in one of 256 terms of a sum, from which the rows drift; most steps agree far more closely."""
