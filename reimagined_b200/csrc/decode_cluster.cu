@@ -1413,8 +1413,8 @@ bool decode_cluster_shape(const tbl_decode_model& m, int batch, int capacity, Cl
             rows = (batch + waves * most - 1) / (waves * most);
             L = layout_of(d, rows, ctas, score_len, kRoom);
         }
-        // limits: shared memory, the fields of the table of pieces, an mbarrier's byte count
-        if (d.inner > 32768 || d.ff > 32768 || L.total > kRoom || L.acc_stride > 32767 || L.x1 - L.x0 > 1 << 19 || L.codes - L.x1 > 1 << 19) continue;
+        // limits: what the separate launches refuse, shared memory, the fields of the table of pieces, an mbarrier's byte count
+        if (d.inner > 16 * 1024 || d.ff > 32768 || L.total > kRoom || L.acc_stride > 32767 || L.x1 - L.x0 > 1 << 19 || L.codes - L.x1 > 1 << 19) continue;
         shape->ctas = ctas; shape->rows = rows; shape->clusters = (batch + rows - 1) / rows; shape->smem = L.total;
         return true;
     }
