@@ -79,6 +79,21 @@ def test_residual_stream_wider_than_the_channels(cuda, tbl, width, rows, in_clus
     assert (clusters.capture() <= 5) == in_clusters
 
 
+@pytest.mark.parametrize("inner,taken", [(16384, True), (16640, False)])
+def test_more_channels_than_a_step_takes(cuda, tbl, inner, taken):
+    """Refused by either route."""
+    import gpu_helpers as H
+    cfg = dict(BASE, mamba_expand=Inner(inner), num_layers=1, attention_period=9)
+    _, clusters, general = engines(cfg, 1, 8)
+    for engine in (clusters, general):
+        if taken:
+            engine.step([5])
+        else:
+            with pytest.raises(Exception, match="tbl_decode_step"):
+                engine.step([5])
+    assert H.device_status() == 0 and (not taken or cuda.equal(clusters.logits, general.logits))
+
+
 def test_long_context_matches_separate_launches_to_rounding(cuda, tbl):
     """300 cached tokens: keys read by four lanes a token.  Scores in another order of sums, 1e-6 of their size, now and then move an 8-bit code by a
     step: 1 / 127 of the row's largest value in one of 256 terms of a sum, from which the rows drift; most steps agree far more closely."""
