@@ -7,7 +7,7 @@
 // shared memory by st.async, which counts its bytes on the receiver's mbarrier -- no launch, no trip through L2, no grid-wide barrier.
 // Clusters share nothing but the weights, so a batch is as many clusters as it needs.  D768, 16 blocks, us a step with the head, separate launches and
 // this: batch 1 323 and 170, 8 422 and 250, 16 416 and 271, 32 551 and 361, 64 667 and 512 (64 cached tokens); 1 344 and 187, 64 811 and 766 (900).
-// The results are the same bit for bit, but for dot products over more than 256 cached tokens.
+// The results are the same bit for bit, but for the attention over more than 256 cached tokens, whose dot products and sums of values are taken in another order.
 //
 // Passes of a block (the row each of them reads is normed and quantised by every CTA for itself, with the arithmetic of the kernels
 // in decode.cu and gemv_strip.cu):
@@ -704,7 +704,8 @@ __device__ __noinline__ void attend(const Params& P, Static& S, const Block& b, 
         for (int w = 1; w < 8; ++w) total += S.red[(row < R ? row : 0) * kMaxParts + w];
         const float inv_sum = __fdiv_rn(1.0f, fmaxf(total, 1e-9f));
         // Its groups of dim / 4 threads take the tokens round-robin, and their sums are added in order: so do ours, in rounds where we have fewer.  (Over a
-        // long context our own groups: 64 sequences with 900 tokens 740 us a step, as against 847 in its order and 812 as separate launches.)
+        // long context our own groups: 64 sequences with 900 tokens 740 us a step, as against 847 in its order and 812 as separate launches.  These are
+        // fewer, and longer sums err more: so eight tokens are added up by themselves, and a sum errs a little less than in its order instead of three times.)
         const int row_threads = dim / 4, groups = nthr / row_threads, all = 256 / row_threads;
         const int its_groups = long_context ? groups : all, g0 = lr / row_threads, d4 = lr - g0 * row_threads;
         const int hold = P.L.partial_all ? max(all, groups) : groups, rounds = (max(all, groups) + hold - 1) / hold;       // groups' sums there is room for
@@ -719,6 +720,7 @@ __device__ __noinline__ void attend(const Params& P, Static& S, const Block& b, 
                 for (int local = g0; local < n_groups; local += groups) {
                     const int g = round * hold + local;
                     float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (long_context) mine[local * row_threads + d4] = o;
                     auto add = [&](const float4& v, float p) {
                         o.x = __fadd_rn(o.x, __fmul_rn(p, v.x)); o.y = __fadd_rn(o.y, __fmul_rn(p, v.y));
                         o.z = __fadd_rn(o.z, __fmul_rn(p, v.z)); o.w = __fadd_rn(o.w, __fmul_rn(p, v.w));
@@ -734,8 +736,13 @@ __device__ __noinline__ void attend(const Params& P, Static& S, const Block& b, 
 #pragma unroll
                         for (int j = 0; j < kInFlight; ++j)
                             if (t + j * its_groups < cached) add(v[j], __fmul_rn(sc[t + j * its_groups - first], inv_sum));
+                        if (long_context) {
+                            float4& sum = mine[local * row_threads + d4];        // (in shared memory: there are no registers to spare)
+                            sum = make_float4(__fadd_rn(sum.x, o.x), __fadd_rn(sum.y, o.y), __fadd_rn(sum.z, o.z), __fadd_rn(sum.w, o.w));
+                            o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        }
                     }
-                    mine[local * row_threads + d4] = o;
+                    if (!long_context) mine[local * row_threads + d4] = o;
                 }
             }
             __syncthreads();
