@@ -14,6 +14,8 @@
 // TMEM is released.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "shares.cuh"
 #include "stack.cuh"
 #include "tc05.cuh"
@@ -46,6 +48,7 @@ struct Params {
     int tiles_m, tiles_n;
     int split;              // shares of K = CTAs of a cluster (SHARED kernel)
     int deep;               // 64 rows: all of an SM's shared memory for one CTA
+    int part;               // 64 rows: blocks of K that are added up in the tensor cores' accumulators
     int vec;                // outputs (and residual) take 4-column vector accesses
     int* status;
 };
@@ -119,6 +122,9 @@ __device__ __forceinline__ void store_block(const Params& p, const uint8_t* stag
 // has twice the stages.  us before | after at 64 rows, cold weights: 24576 gated x 4096 53.2 | 43.1, 32000 x 4096 53.9 | 47.3, 8192 x 4096 18.9 | 17.4,
 // 4096 x 12288 24.6 | 23.2, 2048 x 6144 13.2 | 10.8, 10304 x 2048 15.4 | 12.1.  A step of 64 sequences of the width-4096 Guselix 803 | 762, of 32 of the
 // width-2048 Goguvik 577 | 523, of 24 of the width-2048 Guselix 746 | 642.
+// The accumulators drop the bits that they shift out, which adds up with K (1.1e-9 of the result per number of K).  Few rows have no shares of K to speak of,
+// and went through a kernel that cuts K into eight before; so the accumulators hold a part of K at a time, in two buffers, and the epilogue's warps add the
+// parts up in registers, rounding to nearest.  TMEM is free for the next tile before this one is stored.
 template <int BN, int AR, bool RES, bool SHARED>
 __global__ void __launch_bounds__(threads_for(AR), AR == BM ? 1 : 2)
 dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ Params p) {
@@ -188,6 +194,36 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     // of the width-2048 one 718 and 606).
     if (AR != BM && p.c.M > 16) pdl_launch_dependents();
 
+    const int part = AR == BM ? kblocks : p.part;
+    // 64 rows: waits for the parts of a tile one after the other and adds up `blocks` blocks of 32 columns, `step` apart from `col` on, of this warp's
+    // rows.  False: a wait ran out.
+    auto add_parts = [&](auto& v, int col, int step, int blocks, int& local) {
+        constexpr int kBlocks = sizeof(v) / sizeof(v[0]);
+#pragma unroll
+        for (int i = 0; i < kBlocks; ++i)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) v[i][e] = 0.0f;
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + col;
+        for (int begin = 0; begin < kblocks; begin += part, ++local) {
+            const int buf = local & 1;
+            const bool alive = mbar_wait_bounded(&tmem_full[buf], (local >> 1) & 1, p.status);
+            if (!__all_sync(0xffffffffu, alive)) return false;
+            tc_fence_after();
+#pragma unroll
+            for (int i = 0; i < kBlocks; ++i) {
+                if (i >= blocks) break;
+                uint32_t r[32];
+                tmem_ld32(t_row + buf * BN + i * step, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) v[i][e] += __uint_as_float(r[e]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+        }
+        return true;
+    };
     if (warp == kLoadWarp) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
@@ -214,51 +250,106 @@ dense_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (elect_one()) {
             const uint32_t idesc = idesc_bf16(BN);
             const uint64_t a_desc = smem_desc_sw128(smem_u32(smem)), b_desc = smem_desc_sw128(smem_u32(smem) + kABytes);
-            int s = 0, local = 0, row0, tn;
+            int s = 0, local = 0, row0, tn;                    // local: parts of tiles so far
             uint32_t phase = 0;
             bool alive = true;
-            for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride, ++local) {
-                const int buf = local & 1;
-                if (local >= 2) {
-                    alive = mbar_wait_bounded(&tmem_empty[buf], ((local >> 1) - 1) & 1, p.status);
-                    if (!alive) break;
-                }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    alive = mbar_wait_bounded(&full[s], phase, p.status);
-                    if (!alive) break;
+            for (int tile = first; alive && decode_tile(p, tile, row0, tn); tile += stride) {
+                for (int begin = 0; alive && begin < kblocks; begin += part, ++local) {
+                    const int buf = local & 1, end = min(kblocks, begin + part);
+                    if (local >= 2) {
+                        alive = mbar_wait_bounded(&tmem_empty[buf], ((local >> 1) - 1) & 1, p.status);
+                        if (!alive) break;
+                    }
                     tc_fence_after();
-                    const uint32_t at = static_cast<uint32_t>(s) * (kStageBytes >> 4);     // descriptors count 16 bytes
+                    const uint32_t d_tmem = tmem_base + buf * BN;
+                    for (int kb = begin; kb < end; ++kb) {
+                        alive = mbar_wait_bounded(&full[s], phase, p.status);
+                        if (!alive) break;
+                        tc_fence_after();
+                        const uint32_t at = static_cast<uint32_t>(s) * (kStageBytes >> 4);     // descriptors count 16 bytes
 #pragma unroll
-                    for (int kk = 0; kk < BKB / 32; ++kk) umma_f16(d_tmem, a_desc + at + 2 * kk, b_desc + at + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
-                    umma_commit(&empty[s]);
-                    if (++s == kStages) { s = 0; phase ^= 1; }
+                        for (int kk = 0; kk < BKB / 32; ++kk)
+                            umma_f16(d_tmem, a_desc + at + 2 * kk, b_desc + at + 2 * kk, idesc, ((kb - begin) | kk) != 0 ? 1u : 0u);
+                        umma_commit(&empty[s]);
+                        if (++s == kStages) { s = 0; phase ^= 1; }
+                    }
+                    if (alive) umma_commit(&tmem_full[buf]);
                 }
-                if (alive) umma_commit(&tmem_full[buf]);
             }
         }
     } else if (SHARED) {
         // ---------------- sums of this share into the place of the stages (all of which the MMAs have read) ----------------
         const int quarter = warp & 3, half = AR == BM ? (warp - 2) >> 2 : warp >> 2;
         float* row = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * LDS + half * (BN / 2);
-        bool alive = mbar_wait_bounded(&tmem_full[0], 0, p.status);     // (no share is empty: K has four blocks for each)
-        alive = __all_sync(0xffffffffu, alive);
-        tc_fence_after();
+        if constexpr (AR == BM) {
+            bool alive = mbar_wait_bounded(&tmem_full[0], 0, p.status);     // (no share is empty: K has four blocks for each)
+            alive = __all_sync(0xffffffffu, alive);
+            tc_fence_after();
 #pragma unroll
-        for (int j = 0; j < BN / 2; j += 32) {
-            uint32_t r[32];
-            tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2) + j, r);
-            tmem_ld_wait();
-            if (alive)
+            for (int j = 0; j < BN / 2; j += 32) {
+                uint32_t r[32];
+                tmem_ld32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2) + j, r);
+                tmem_ld_wait();
+                if (alive)
 #pragma unroll
-                for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(row + j + e) = make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);
+                    for (int e = 0; e < 32; e += 4) *reinterpret_cast<uint4*>(row + j + e) = make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);
+            }
+        } else {
+            float v[BN / 64][32];
+            int local = 0;
+            if (add_parts(v, half * (BN / 2), 32, BN / 64, local))
+#pragma unroll
+                for (int i = 0; i < BN / 64; ++i)
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4*>(row + 32 * i + e) = make_float4(v[i][e], v[i][e + 1], v[i][e + 2], v[i][e + 3]);
+        }
+    } else if constexpr (AR != BM) {
+        // ---------------- epilogue warps, 64 rows ----------------
+        // Two blocks of 32 columns a warp: of a gated layer a pair, else every other one.  TMEM is free again before anything is stored.
+        const int quarter = warp & 3, half = warp >> 2;
+        uint8_t* stage = epi_stage + (2 * half + quarter) * 4096;
+        const bool pair = p.c.pair_cols > 0;
+        const Activation act = activation_of(p.c.act);
+        int local = 0, tile_row0, tn;
+        for (int tile = first; decode_tile(p, tile, tile_row0, tn); tile += stride) {
+            const int row0 = tile_row0 + quarter * 32, valid = min(32, p.c.M - row0);
+            const int nblocks = min(BN / 32, (p.c.N - tn * BN + 31) / 32), b0 = pair ? 2 * half : half, step = pair ? 1 : 2;
+            const int mine = valid <= 0 || b0 >= nblocks ? 0 : (b0 + step < nblocks ? 2 : 1);
+            float v[2][32];
+            if (!add_parts(v, 32 * b0, 32 * step, mine, local)) break;
+            const int n0 = tn * BN + 32 * b0;
+            if (pair && mine) {                                // (N is a multiple of 64: both blocks are there)
+                const float bias_l = p.c.bias ? __ldg(p.c.bias + n0 + lane) : 0.0f, bias_u = p.c.bias ? __ldg(p.c.bias + n0 + 32 + lane) : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const float g = v[0][i] + __shfl_sync(0xffffffffu, bias_l, i), u = v[1][i] + __shfl_sync(0xffffffffu, bias_u, i);
+                    v[0][i] = activate(act, g) * u;
+                }
+            }
+#pragma unroll 1
+            for (int b = 0; b < (pair ? mine / 2 : mine); ++b) {
+                const int col = n0 + 64 * b;
+                if (p.c.bias && !pair) {
+                    const float bias = col + lane < p.c.N ? __ldg(p.c.bias + col + lane) : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) v[0][i] += __shfl_sync(0xffffffffu, bias, i);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    *reinterpret_cast<float4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                        make_float4(v[0][4 * j], v[0][4 * j + 1], v[0][4 * j + 2], v[0][4 * j + 3]);
+                __syncwarp();
+                store_block<RES>(p, stage, lane, row0, valid, pair ? col >> 1 : col, pair ? p.c.pair_cols : p.c.N);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[0][i] = v[1][i];
+            }
         }
     } else {
         // ---------------- epilogue warps ----------------
         const int quarter = warp & 3;          // TMEM lanes 32*quarter .. +31 are this warp's
-        const int half = AR == BM ? (warp - 2) >> 2 : warp >> 2;      // which of the two warps of the quarter
-        uint8_t* stage = epi_stage + (AR == BM ? warp - 2 : 2 * half + quarter) * 4096;
+        const int half = (warp - 2) >> 2;      // which of the two warps of the quarter
+        uint8_t* stage = epi_stage + (warp - 2) * 4096;
         const bool pair = p.c.pair_cols > 0;
         const Activation act = activation_of(p.c.act);
         int local = 0, tile_row0, tn;
@@ -411,6 +502,11 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
                 if (best == 0.0 || us < best) { best = us; bn = b; split = s; p.deep = deep; }
             }
         }
+        // Blocks of K that the accumulators take at a time: eight, and no more than a warp of the row-streaming kernel has where that is the other choice.
+        // us and error against 64 bits at 4, 8 and all blocks: 64 x 24576 gated x 4096 38.1, 37.8, 37.8; 64 x 12288 gated x 2048 16.1, 15.4, 14.9;
+        // 64 x 6208 x 4096 15.0, 14.7, 14.5 and 2.4e-7, 4.7e-7, 2.1e-6; 64 x 10368 x 2048 13.2, 12.0, 11.3; 16 x 32000 x 4096 43.7, 43.6, 43.6 and 2.4e-7, 4.8e-7, 4.4e-6.
+        const bool rows_too = c.M <= 16 || (c.M <= 32 && c.N <= 4096) || (c.M <= 48 && c.N <= 2048);
+        p.part = rows_too ? static_cast<int>(std::min(8LL, std::max(2LL, kb / 8))) : 8;
     } else {
         // More than 64 rows: tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
         // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to

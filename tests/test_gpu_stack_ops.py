@@ -197,6 +197,50 @@ def test_dense_route_of_few_rows(cuda, stack_lib, m, k, n, route):
     assert torch.equal(outs[0], outs[route]) and not torch.equal(outs[TENSOR], outs[ROWS])
 
 
+@pytest.mark.parametrize("m,k,n", [(9, 3072, 15552), (16, 4096, 20736), (12, 2048, 7105), (16, 4104, 8288), (9, 12288, 4096), (17, 1024, 4096), (24, 3072, 1024),
+                                   (32, 4088, 2040), (33, 1024, 1024), (48, 1528, 2048), (48, 1024, 72)])
+def test_dense_of_few_rows_errs_no_more_than_streaming(cuda, stack_lib, m, k, n):
+    """Where the GEMM takes over from the row-streaming kernel: it is no further from 64 bits (5 %: both errors are those of one draw)."""
+    torch = cuda
+    torch.manual_seed(n)
+    b = Buf(torch)
+    x, w = torch.randn(m, k).bfloat16().cuda(), torch.randn(n, k).bfloat16()
+    view, errs = b.view(w), []
+    want = x.double() @ w.cuda().double().T
+    for r in (0, ROWS):
+        out = torch.full((m, n), float("nan"), device="cuda")
+        assert stack_lib.tbl_dense_forward(C.byref(view), 1, r, x.data_ptr(), k, m, None, out.data_ptr(), stream(torch)) == 0
+        errs.append(float(((out.double() - want).square().sum() / want.square().sum()).sqrt()))
+    assert errs[0] <= 1.05 * errs[1] < 5e-6, errs
+
+
+@pytest.mark.parametrize("m,k,n,ff", [(64, 64, 128, 64), (64, 512, 64, 32), (63, 520, 200, 64), (17, 576, 72, 40), (64, 1024, 148 * 128 * 2 + 8, 148 * 64 + 32), (40, 1032, 148 * 64 * 2 + 1, 200),
+                                      (1, 4104, 130, 33), (64, 4096, 6208, 3104), (33, 16392, 256, 100), (64, 1032, 148 * 128 * 4 + 65, 148 * 64 * 4 + 7)])
+def test_dense_of_few_rows_in_parts_of_k(cuda, stack_lib, m, k, n, ff):
+    """Up to 64 rows: one part of K and many, with a short last one and a short last block; one tile a block and several (buffers used again across tiles);
+    shares of K; bias, residual and gate.  A part is 512 of K or less: 1.1e-9 of a result per number of K in it, and half of 2^-24 a sum of parts."""
+    from reimagined_b200.stack import StackEngine
+    torch, rng = cuda, np.random.default_rng(n)
+    torch.manual_seed(k)
+    b = Buf(torch)
+    x, w = torch.randn(m, k).bfloat16().cuda(), (torch.randn(n, k) * k ** -0.5).bfloat16()
+    bias = rng.standard_normal(n)
+    want = x.double() @ w.cuda().double().T
+    plain, out = torch.full((m, n), float("nan"), device="cuda"), torch.randn(m, n, device="cuda")
+    full = want + torch.as_tensor(np.float32(bias)).cuda().double() + out.double()
+    assert stack_lib.tbl_dense_forward(C.byref(b.view(w)), 1, TENSOR, x.data_ptr(), k, m, None, plain.data_ptr(), stream(torch)) == 0
+    assert stack_lib.tbl_dense_forward(C.byref(b.view(w, bias)), 1, TENSOR, x.data_ptr(), k, m, out.data_ptr(), out.data_ptr(), stream(torch)) == 0
+    rms = lambda d, of: float((d.square().sum() / of.square().sum()).sqrt())
+    assert rms(plain.double() - want, want) <= 7e-7 and rms(out.double() - full, full) <= 7e-7
+    gate, up = ((torch.randn(ff, k) * k ** -0.5).bfloat16() for _ in range(2))
+    h = torch.full((m, ff), float("nan"), device="cuda", dtype=torch.bfloat16)
+    assert stack_lib.tbl_gated_dense_forward(C.byref(b.view(StackEngine._paired(None, gate, up))), 1, TENSOR, x.data_ptr(), k, m, ff, h.data_ptr(),
+                                             stream(torch)) == 0
+    gw, uw = (x.double() @ v.cuda().double().T for v in (gate, up))
+    assert_close(f64(h), (torch.nn.functional.silu(gw) * uw).cpu().numpy(), 4e-3)
+    assert stack_lib.tbl_device_status(stream(torch)) == 0
+
+
 @pytest.mark.parametrize("route,precision", [(SIMT, 0), (GEMV, 0), (GEMV, 1), (SIMT, 1), (TENSOR, 1), (ROWS, 1)])
 @pytest.mark.parametrize("m,k,ff", [(9, 512, 70), (1, 64, 32), (3, 40, 37), (4, 128, 200), (1, 1024, 3000), (150, 72, 100), (260, 136, 333)])
 def test_gated_dense(cuda, stack_lib, route, precision, m, k, ff):
