@@ -1391,6 +1391,18 @@ int clusters_at_once(int ctas) {
     return k = n;
 }
 
+// Whether clusters of this shape still pay over `len` cached tokens.  Here a CTA attends for its heads and all its cluster's sequences, by itself; separate
+// launches have a block per head and sequence, on every SM: us a cached token on the busiest SM, by 64-wide heads, fitted to widths of 256 to 2048, batches
+// of 1 to 256 and 64 to 10000 tokens.  Against that stands what a step over few tokens is shorter by, a block: 10 to 14 us, 18 to 30 from width 1024 on where
+// a CTA's share of the weights is small; past 64 sequences 50 and more, 23 to 50.  us a step, clusters and launches, width 768, 16 blocks of which two
+// attend: 64 sequences, 1084 tokens 807 and 848, 1284 864 and 866, 2000 1082 and 973, 3000 1377 and 1123; 48, 1684 740 and 816, 3000 981 and 959; 32, 2584 759 and 780,
+// 3000 823 and 814.  A cache is taken to be as full as it can get: a step's positions are on the device.
+bool context_pays(const Dims& d, int rows, int ctas, int waves, int batch, int len, int attending, int n_blocks, long long share) {
+    const double heads = d.head_dim / 64.0, here = 0.0145 * rows * ((d.a_heads + ctas - 1) / ctas) * waves * heads, there = 0.0175 + 7.2e-5 * batch * d.a_heads * heads;
+    const double lead = batch > 64 ? (d.D >= 1024 ? 25.0 : 50.0) : (d.D >= 1024 && share <= 256 * 1024 ? 18.0 : 10.0);
+    return attending * len * (here - there) <= lead * n_blocks;
+}
+
 // Clusters of sixteen CTAs (seven at once on a B200, up to eight sequences each) where they hold the batch, else of eight (fifteen at once); as few
 // sequences a cluster as lets all run at once.  A CTA streams its share of the weights by itself, so that wide models are better off with every SM at
 // every matrix, one launch each: us a step of 8 blocks at batch 1 / 7 / 16, this kernel and separate launches, by width: 1536 256 / 271 / 284 and 330 / 407 /
@@ -1399,8 +1411,9 @@ int clusters_at_once(int ctas) {
 // clusters only where the separate launches leave their GEMV and GEMM of up to 64 rows (768: batch 100 680 and 1841, batch 1024 7018 and 16807).
 bool decode_cluster_shape(const tbl_decode_model& m, int batch, int capacity, ClusterShape* shape) {
     Dims d;
-    int score_len;
+    int score_len, attending = 0;
     if (!common_dims(m, capacity, &d, &score_len)) return false;
+    for (int i = 0; i < m.n_blocks; ++i) attending += m.blocks[i].hybrid != 0;
     // the parts that gemv_strip_kernel takes a row's sum of squares in: more than sum_parts() has places for
     if (batch <= gemv_strip_fused_rows(d.D) && sum_strips_parts(d.D) > kStripParts) return false;
     for (int ctas = 16; ctas >= 8; ctas >>= 1) {
@@ -1422,6 +1435,7 @@ bool decode_cluster_shape(const tbl_decode_model& m, int batch, int capacity, Cl
         }
         // limits: what the separate launches refuse, shared memory, the fields of the table of pieces, an mbarrier's byte count
         if (d.inner > 16 * 1024 || d.ff > 32768 || L.total > kRoom || L.acc_stride > 32767 || L.x1 - L.x0 > 1 << 19 || L.codes - L.x1 > 1 << 19) continue;
+        if (!context_pays(d, rows, ctas, waves, batch, score_len, attending, m.n_blocks, share)) continue;
         shape->ctas = ctas; shape->rows = rows; shape->clusters = (batch + rows - 1) / rows; shape->smem = L.total;
         return true;
     }

@@ -198,6 +198,25 @@ def test_value_sums_over_a_long_context(cuda, tbl, change, rows):
     assert clusters.capture() <= 6 < general.capture()
 
 
+@pytest.mark.parametrize("change,rows,short,beyond", [
+    (dict(num_layers=1, attention_period=1, attention_slot=0), 64, 250, 300),          # every block attends
+    ({}, 64, 2100, 2300),                                        # one block of eight
+    (dict(n_heads=2, n_kv_heads=1), 64, 700, 800),               # heads twice as wide
+    ({}, 1, 4000, None),                                         # one sequence: nowhere
+])
+def test_route_by_the_context(cuda, tbl, change, rows, short, beyond):
+    """Clusters where they are faster over as many tokens as the cache takes, or the window lets a step see; either way the same logits."""
+    import gpu_helpers as H
+    cfg = dict(BASE, **change)
+    for capacity, window, in_clusters in [(short, 4096, True), *([(beyond, 4096, False), (beyond, short, True), (short, beyond, True)] if beyond else [])]:
+        _, clusters, general = engines(cfg, rows, capacity, window)
+        ids = np.random.default_rng(rows).integers(0, cfg["vocab_size"], rows).tolist()
+        for _ in range(2):
+            assert cuda.equal(clusters.step(ids), general.step(ids)), (capacity, window)
+        assert (clusters.capture() <= 6) == in_clusters, (capacity, window)
+    assert H.device_status() == 0
+
+
 def test_long_context_matches_separate_launches_to_rounding(cuda, tbl):
     """300 cached tokens: keys read by four lanes a token.  Scores in another order of sums, 1e-6 of their size, now and then move an 8-bit code by a
     step: 1 / 127 of the row's largest value in one of 256 terms of a sum, from which the rows drift; most steps agree far more closely."""
