@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(32 * kQuarters * MAPS) attention_stream_kernel
         }
     __syncthreads();
     // With more than one block to an SM these leave no room on theirs, and up to 16 rows the output projection's blocks (dense_rows.cu) would crowd onto the SMs
-    // that have none: they come when these are done (16 sequences of the width-4096 Goguvik: a step 774 and 620 us).  More rows are the GEMM's, one block an SM,
-    // whom it helps to come early (64 sequences 653 and 637 us), as it helps where every SM has room (8 sequences of width 2048: 448 and 436).
+    // that have none: they come when these are done (16 sequences of the width-4096 Goguvik: a step 774 and 620 us).  More rows are the GEMM's, whom it helps
+    // to come early although two of its blocks share an SM (a step without and with: 64 sequences of width 4096 567 and 563 us, 32 494 and 485, 64 of width 2048
+    // 555 and 547; 24 of width 2048 561 and 562), as it helps where every SM has room (8 sequences of width 2048: 448 and 436).
     if (gridDim.x * gridDim.y * gridDim.z <= kNumSm || gridDim.x / p.G * p.n_tok > 16) pdl_launch_dependents();
     // the quarters come together: sums of this split, a warp per row
     const size_t quarter_step = static_cast<size_t>(MAPS) * kRows * p.vp;

@@ -6,7 +6,7 @@
 // its own: a projection's rows are spread over the CTAs, and a row that the next projection reads as a whole is gathered into every CTA's
 // shared memory by st.async, which counts its bytes on the receiver's mbarrier -- no launch, no trip through L2, no grid-wide barrier.
 // Clusters share nothing but the weights, so a batch is as many clusters as it needs.  D768, 16 blocks, us a step with the head, separate launches and
-// this: batch 1 323 and 170, 8 422 and 250, 16 416 and 271, 32 551 and 361, 64 667 and 512 (64 cached tokens); 1 344 and 187, 64 811 and 766 (900).
+// this: batch 1 318 and 173, 8 417 and 248, 16 408 and 263, 32 530 and 361, 64 649 and 494 (64 cached tokens); 1 338 and 188, 64 819 and 745 (900).
 // The results are the same bit for bit, but for the attention over more than 256 cached tokens, whose dot products and sums of values are taken in another order.
 //
 // Passes of a block (the row each of them reads is normed and quantised by every CTA for itself, with the arithmetic of the kernels
@@ -1407,7 +1407,7 @@ bool context_pays(const Dims& d, int rows, int ctas, int waves, int batch, int l
 // sequences a cluster as lets all run at once.  A CTA streams its share of the weights by itself, so that wide models are better off with every SM at
 // every matrix, one launch each: us a step of 8 blocks at batch 1 / 7 / 16, this kernel and separate launches, by width: 1536 256 / 271 / 284 and 330 / 407 /
 // 490; 2048 359 / 347 / 386 and 421 / 556 / 619; 3072 735 / 674 / 2799 and 706 / 759 / 844; 4096 1263 / 1131 / - and 869 / 944 / 1065; in clusters of
-// eight, batch 64: 1024 (16 blocks) 659 and 954, 1536 871 and 609.  Hence the line at 400 KB of a block's three large matrices.  Several waves of
+// eight, 60 sequences of 1024 290 and 442, 40 of 1280 378 and 468, 64 of 1536 871 and 609.  Hence the line at 400 KB of a block's three large matrices.  Several waves of
 // clusters only where the separate launches leave their GEMV and GEMM of up to 64 rows (768: batch 100 680 and 1841, batch 1024 7018 and 16807).
 bool decode_cluster_shape(const tbl_decode_model& m, int batch, int capacity, ClusterShape* shape) {
     Dims d;

@@ -244,9 +244,12 @@ bool gemv_supported(const DenseCall& c) {
 }
 
 // Streaming the weights through warp-level MMAs beats the tcgen05 GEMM up to 8 rows.  Up to 16 it does for gated layers (us, rows and GEMM: 16 x 12288 x 2048
-// 12.4 and 18 .. 23, 24576 x 4096 41 and 43) and except where, with some K, the matrix is very tall (16 x 16384 x 2048 25.8 and 20.1, 32000 x 4096 86 and 46;
-// but 10304 x 2048 13.6 and 17.0) or its blocks are a little more than a wave of three to an SM (N of 7105 .. 8288: 8192 x 4096 24.6 and 15.6, 8192 x 2048 14.2
-// and 11.6; but 8192 x 1024 8.8 and 8.7), or where K is long beside N, which the GEMM shares out (4096 x 12288 32 and 22).  A step with the first two: 16
+// 12.4 and 18 .. 23, 24576 x 4096 41 and 43) and except where, with some K, the matrix is very tall, which is another wave of blocks (9 and 16 x 14336 x 2048
+// 23.5 and 22.0, 24.2 and 20.9, 16384 23.1 and 22.0, 24.4 and 21.2, 20480 23.9 and 23.5, 25.3 and 21.6; 16 x 14336 x 4096 44 and 23, 32000 82 and 44; but 14208 x
+// 2048 14.7 and 22.2, 15.2 and 21.0, 10304 12.9 and 20.2, 13.4 and 18.9), or its blocks are a little more than a wave of three to an SM (N of 7105 .. 8288, 9 and 16
+// rows: 7168 x 2304 13.4 and 10.6, 14.1 and 11.2; 8192 x 2560 15.7 and 12.1, 16.4 and 12.3; 8288 x 3072 17.8 and 16.3, 18.9 and 15.8; 7680 x 4096 22.6 and 14.4,
+// 23.7 and 14.8; at K of 2048 as long, 12.5 .. 13.7 and 11.6 .. 13.4; but 8192 x 1024 8.8 and 8.7), or where K is long beside N, which the GEMM shares out
+// (4096 x 12288 32 and 22).  (The GEMM's times vary by up to a fourth with where the activations lie.)  A step with the first two: 16
 // sequences of the width-4096 Guselix 714 and 627, of width 3072 500 and 459, 10 of the width-4096 Goguvik 577 and 535.  Lines that only the layers by
 // themselves bear out are not drawn: 4096 x 4096 takes 13.0 and 11.4, steps with it by the GEMM are up to a fourth longer, and 32000 x 1024 26 and 17, but
 // steps 2 % longer.

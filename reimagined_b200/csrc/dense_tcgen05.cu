@@ -479,7 +479,7 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     p.vec = (cols % 4 == 0) && (c.ldo % 4 == 0) && (reinterpret_cast<uintptr_t>(c.out_f32) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(c.out_b16) & 7) == 0 && (reinterpret_cast<uintptr_t>(c.residual) & 15) == 0;
     const long long tm = (c.M + BM - 1) / BM, kb = (c.K + BKE - 1) / BKE;
-    const int a_rows = c.M < 64 ? 64 : (c.M < BM ? static_cast<int>(c.M) : BM);
+    const int a_rows = c.M < BM ? static_cast<int>(c.M) : BM;         // (more than 64)
     int bn = 64, split = 1;
     double best = 0.0;
     if (c.M <= 64) {
@@ -510,9 +510,9 @@ cudaError_t launch_dense_tensor(const DenseCall& c, cudaStream_t st) {
     } else {
         // More than 64 rows: tile width and shares of K by the blocks of K that a CTA takes one after another (an SM takes in about 100 GB/s, and
         // 0.12 us pass all the same) against what it costs to exchange the sums of shared tiles; constants in us, fitted to
-        // measurements.  64 x 12288 x 4096: 64 tiles of 64 columns took 62 us, 32 of 128 in four shares 23; 512 x 6144 x 2048:
-        // 33 and 19; 128 x 3072 x 3072: 19 and 11; 900 x 2048 x 2048: 15 alone, 19 shared.  192 columns, whole tiles only, where 256 leave much of a last wave
-        // empty and 128 take one more (64 rows of the width-4096 model: 16 tokens 0.6 % shorter; 900-token prompts at width 2048: 0.7 %).
+        // measurements.  Whole and shared: 512 x 2048 x 6144 33 and 19; 128 x 3072 x 3072 19 and 11; 900 x 2048 x 2048 15 and 19.  192 columns, whole tiles only,
+        // where 256 leave much of a last wave empty and 128 take one more (us without and with: 900 x 10368 x 2048 41.3 and 38.4, 900 x 3072 x 3072 22.5 and 19.7,
+        // 251 x 20736 x 4096 58.9 and 53.6, 512 x 5184 x 1024 11.6 and 10.0, 100 x 24576 gated x 4096 42.4 and 41.3).
         for (const int b : {256, 192, 128, 64}) {
             if (b > 64 && c.N <= b / 2) continue;
             const long long tiles = tm * ((c.N + b - 1) / b);

@@ -237,7 +237,7 @@ def test_long_context_matches_separate_launches_to_rounding(cuda, tbl):
 
 
 def test_clusters_match_the_oracle_through_a_long_window(cuda, port, tbl):
-    """Sliding window shorter than the reply, positions that differ from what the cache holds, and a cache that runs full."""
+    """Sliding window shorter than the reply, and a cache that runs full."""
     import gpu_helpers as H
     from oracle.decode import PortDecoder
     cfg = dict(BASE)
